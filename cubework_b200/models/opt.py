@@ -4,8 +4,9 @@ Parity: benchmark/opt/opt.py:20-653 — vocab-parallel token embedding, learned 
 offset-2 table indexed by the running count of non-pad tokens (:20-40), pre-LN (or post-LN for the
 350m layout) decoder layers with packed per-head QKV, ReLU FFN, tied LM head, shifted LM loss, KV
 cache for incremental decoding, presets ``opt_125m ... opt_175b`` (``opt_13b``: hidden 5120, ffn 20480,
-40 layers, 64 heads).  Training attention is the fused causal kernel; the incremental-decoding path
-(a few query rows against a cache) uses the plain formulation.
+40 layers, 64 heads).  Training attention and, under autocast, that of a cached prompt is the fused causal
+kernel; one further token appends to the cache and attends over it in one kernel; other cached calls use
+the plain formulation.
 """
 import torch
 import torch.nn as nn
@@ -48,7 +49,14 @@ class OPTAttention(SelfAttention):
         qkv = self.query_key_value(x)
         b, t, w = qkv.shape
         heads = w // (3 * self.head_dim)
-        q, k, v = qkv.view(b, t, heads, 3 * self.head_dim).permute(0, 2, 1, 3).chunk(3, dim=-1)
+        packed = qkv.view(b, t, heads, 3 * self.head_dim)
+        if past_key_value is not None and ops.decode_ready(packed, *past_key_value, key_bias):
+            o, k, v = ops.decode_attention(packed, *past_key_value, key_bias)
+            return self.dense(o), (k, v)
+        q, k, v = packed.permute(0, 2, 1, 3).chunk(3, dim=-1)
+        if past_key_value is None and ops.prefill_ready(packed, key_bias):
+            o = ops.attention_packed(packed, True, None if key_bias is None else key_bias.float().contiguous())
+            return self.dense(o), (k, v)
         if past_key_value is not None:
             k = torch.cat([past_key_value[0], k], dim=2)
             v = torch.cat([past_key_value[1], v], dim=2)

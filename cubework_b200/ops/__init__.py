@@ -341,6 +341,49 @@ def attention_with_prob_dropout(qkv: torch.Tensor, causal: bool, key_bias: Optio
     return torch.matmul(p, v).transpose(1, 2).reshape(B, T, H * dh)
 
 
+def _needs_grad(*tensors):
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+
+
+def decode_ready(qkv, k_past, v_past, key_bias) -> bool:
+    """Whether :func:`decode_attention` takes these tensors: one query token, no gradients, 16-bit caches of the
+    projection's dtype with dense 16-byte aligned rows, one bias value per key.  Everything else (several query tokens
+    against a cache, mixed dtypes, head dims that are no multiple of 8) keeps the materialised formulation."""
+    B, T, H, D3 = qkv.shape
+    dh = D3 // 3
+    if T != 1 or dh % 8 or dh > 256 or not use_kernels(qkv) or not qkv.is_contiguous() or qkv.data_ptr() % 16:
+        return False
+    keys = k_past.shape[2] if k_past.dim() == 4 else -1
+    for c in (k_past, v_past):
+        if c.dtype != qkv.dtype or c.device != qkv.device or tuple(c.shape) != (B, H, keys, dh) or c.data_ptr() % 16:
+            return False
+        sb, sh, st, sd = c.stride()
+        if sd != 1 or (sb | sh | st) % 8:
+            return False
+    if key_bias is not None and (key_bias.device != qkv.device or tuple(key_bias.shape) != (B, keys + 1)):
+        return False
+    return not _needs_grad(qkv, k_past, v_past, key_bias)
+
+
+def decode_attention(qkv, k_past, v_past, key_bias=None, scale=None):
+    """One token per sequence: packed ``qkv`` ``[B, 1, heads, 3*dh]`` against caches ``[B, heads, T, dh]``.  Returns
+    ``(out [B, 1, heads*dh], k, v)`` with caches that are one key longer (new tensors; the old ones stay as they are).
+    Scores, probabilities and sums are fp32."""
+    scale = scale if scale is not None else 1.0 / math.sqrt(qkv.shape[-1] // 3)
+    return ext.decode_attention(qkv, k_past, v_past, key_bias, scale)
+
+
+def prefill_ready(qkv, key_bias) -> bool:
+    """Whether a cached prompt may run through :func:`attention_packed`: no gradients, and 16-bit autocast, under which
+    the materialised formulation rounds its scores and probabilities to 16 bits as well (without autocast it keeps
+    them in fp32, and so does this framework)."""
+    B, T, H, D3 = qkv.shape
+    return (use_kernels(qkv) and D3 // 3 <= 128 and torch.is_autocast_enabled("cuda")
+            and torch.get_autocast_dtype("cuda") in _LOWP
+            and (key_bias is None or (key_bias.device == qkv.device and tuple(key_bias.shape) == (B, T)))
+            and not _needs_grad(qkv, key_bias))
+
+
 # ---------------------------------------------------------------------------------------------------
 # embedding
 # ---------------------------------------------------------------------------------------------------

@@ -47,6 +47,9 @@ torch::Tensor attention_bwd(torch::Tensor dout, torch::Tensor qkv, torch::Tensor
                             c10::optional<torch::Tensor> key_bias, double scale, int64_t status_ptr,
                             c10::optional<torch::Tensor> packed, c10::optional<torch::Tensor> trace);
 bool attention_ready();
+// decode_sm100.cu
+std::vector<torch::Tensor> decode_attention(torch::Tensor qkv, torch::Tensor k_past, torch::Tensor v_past,
+                                            c10::optional<torch::Tensor> key_bias, double scale);
 // comm.cu
 void register_comm(pybind11::module& m);
 
@@ -143,6 +146,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("multi_scale", &cw::multi_scale);
   m.def("attention_fwd", &cw::attention_fwd);
   m.def("attention_bwd", &cw::attention_bwd);
+  m.def("decode_attention", &cw::decode_attention);
   m.def("attention_ready", &cw::attention_ready);
   cw::register_comm(m);
 }

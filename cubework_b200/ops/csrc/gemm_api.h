@@ -25,4 +25,8 @@ struct GemmArgs {
 
 void gemm_launch(const GemmArgs& g, cudaStream_t stream);
 
+// y = act(x W^T + b) with at most this many rows of x and a 16-bit output (decode_sm100.cu)
+constexpr int kSkinnyRows = 32;
+void skinny_gemm_launch(const GemmArgs& g, cudaStream_t stream);
+
 }  // namespace cw

@@ -391,6 +391,11 @@ static void dispatch_major(bool ak, bool bk, const CUtensorMap& ta, const CUtens
 
 // Host entry.  a: [M,K] (trans_a=false) or [K,M]; b: [K,N] (trans_b=false) or [N,K]; both contiguous 2-D.
 void gemm_launch(const GemmArgs& g, cudaStream_t stream) {
+  // a handful of rows against row-major weights: the weight-streaming kernel of decode_sm100.cu
+  if (!g.trans_a && g.trans_b && !g.out_f32 && g.M <= kSkinnyRows) {
+    skinny_gemm_launch(g, stream);
+    return;
+  }
   const bool a_kmajor = !g.trans_a;
   const bool b_kmajor = g.trans_b;
   // 128-wide tiles read 128 B of shared memory per tensor-core clock against 96 B for 256-wide ones and lose even

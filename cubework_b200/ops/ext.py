@@ -254,3 +254,8 @@ def attention_bwd(dout, qkv, out, lse, causal, key_bias, scale):
     _count(3 if packed is None else 4)
     return m.attention_bwd(dout, qkv, out, lse, bool(causal), key_bias, float(scale), m.status_device_ptr(), packed,
                            ATTN_TRACE)
+
+
+def decode_attention(qkv, k_past, v_past, key_bias, scale):
+    _count(1)
+    return tuple(require().decode_attention(qkv, k_past, v_past, key_bias, float(scale)))
