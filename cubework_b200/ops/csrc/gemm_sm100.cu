@@ -396,6 +396,11 @@ void gemm_launch(const GemmArgs& g, cudaStream_t stream) {
     skinny_gemm_launch(g, stream);
     return;
   }
+  // large products go to pairs of SMs (gemm_pair_sm100.cu); what follows serves short and narrow ones
+  if (const int pair_splits = gemm_pair_splits(g)) {
+    gemm_pair_launch(g, pair_splits, stream);
+    return;
+  }
   const bool a_kmajor = !g.trans_a;
   const bool b_kmajor = g.trans_b;
   // 128-wide tiles read 128 B of shared memory per tensor-core clock against 96 B for 256-wide ones and lose even

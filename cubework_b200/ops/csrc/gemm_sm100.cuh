@@ -56,6 +56,9 @@ struct GemmParams {
   int* status;        // host-visible error word
 };
 
+int gemm_pair_splits(const GemmArgs& g);                                       // gemm_pair_sm100.cu
+void gemm_pair_launch(const GemmArgs& g, int splits, cudaStream_t stream);
+
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                     const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

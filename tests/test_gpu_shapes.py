@@ -1,0 +1,64 @@
+"""Kernels at the edges of their tiles and dispatch rules: column sums over few and many columns, wide layer norms with a
+residual, the row sums and the dQ conversion of attention, wide heads, and the GEMM on pairs of SMs."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+UNIT = {torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11}     # largest relative error of one rounding (8 / 11 significant bits)
+
+
+def _ops():
+    from cubework_b200 import ops
+    from cubework_b200.ops import ext
+    ext.require()
+    return ops, ext
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("trans_a,trans_b", [(False, True), (False, False), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,K", [
+    (256, 256, 64),            # one tile, one k-block
+    (264, 64, 72),             # a second row block of 8 rows, the narrowest tile
+    (1000, 1608, 200),         # ragged in every extent
+    (4096, 1600, 1600),        # tiles that are not 256 wide
+    (2048, 776, 4104),         # more k-blocks than stages, a ragged last one
+    (33, 50304, 136),          # half of every row block empty
+])
+def test_gemm_on_pairs(dtype, trans_a, trans_b, M, N, K):
+    ops, ext = _ops()
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    pad = lambda n: (n + 7) // 8 * 8
+    M = pad(M) if trans_a else M
+    a = torch.randn((K, M) if trans_a else (M, K), generator=g, device="cuda").to(dtype)
+    b = torch.randn((N, K) if trans_b else (K, N), generator=g, device="cuda").to(dtype)
+    ref = (a.float().t() if trans_a else a.float()) @ (b.float().t() if trans_b else b.float())
+    out32 = ops.gemm(a, b, trans_a, trans_b, out_dtype=torch.float32)
+    out = ops.gemm(a, b, trans_a, trans_b)
+    ext.check_status()
+    assert (out32 - ref).norm() <= 1e-5 * ref.norm()              # both sums are fp32
+    assert ((out.float() - ref).abs() <= UNIT[dtype] * ref.abs() + 1e-4 * math.sqrt(K)).all()
+
+
+@pytest.mark.parametrize("act", [None, "gelu", "relu"])
+@pytest.mark.parametrize("M,N", [(300, 1600), (520, 1000), (4096, 160), (700, 2300), (260, 60)])
+def test_gemm_on_pairs_epilogue(M, N, act):
+    """Bias, activation and the pre-activation copy: whole chunks, half chunks at a tile's or the matrix's end, and a row
+    pitch that TMA cannot store."""
+    ops, ext = _ops()
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randn(M, 264, generator=g, device="cuda").bfloat16()
+    b = (torch.randn(N, 264, generator=g, device="cuda") / 16).bfloat16()
+    bias = torch.randn(N, generator=g, device="cuda")
+    z_ref = a.double() @ b.double().t() + bias.double()
+    y_ref = torch.nn.functional.gelu(z_ref) if act == "gelu" else z_ref.relu() if act == "relu" else z_ref
+    y, z = ext.gemm(a, b, False, True, bias, act, torch.bfloat16, True)
+    y1 = ext.gemm(a, b, False, True, bias, act, torch.bfloat16, False)
+    y32 = ext.gemm(a, b, False, True, bias, act, torch.float32, False)
+    ext.check_status()
+    u = UNIT[torch.bfloat16]
+    assert ((z.double() - z_ref).abs() <= u * z_ref.abs() + 1e-4).all()
+    assert ((y.double() - y_ref).abs() <= u * y_ref.abs() + 1e-4).all() and torch.equal(y, y1)
+    assert ((y32.double() - y_ref).abs() <= 1e-4).all()
