@@ -9,6 +9,7 @@
 #include <c10/cuda/CUDAException.h>
 #include <torch/extension.h>
 
+#include "colsum.cuh"
 #include "common.cuh"
 
 namespace cw {
@@ -119,14 +120,19 @@ __device__ __forceinline__ float gelu_grad_fast(float x) {
   return fmaf(x, 0.3989422804014327f * e, cdf);
 }
 
-// Each CTA owns a stripe of 2048 columns (256 threads x 8) and a range of rows; per-thread column sums stay
-// in registers and are written as partials[blockIdx.y, N].  Two rows are in flight per thread.
-template <typename T, int ACT, bool WRITE_DZ, bool WANT_SUM>
+// A CTA owns a stripe of 8 * TX columns and a range of rows; its 256 / TX row groups take the rows in turn, two at a
+// time.  TX follows from the width (act_stripe): with one stripe of 2048 columns 160 of 256 threads had no column at
+// N = 768 and a quarter of them none at N = 3072 (6304 x 3072, GELU: 36.9 -> 29.1 us; 50432 x 3072: 261 -> 211;
+// 32768 x 6400: 403 -> 320 or 3.9 TB/s, bound by the error function's arithmetic).  Column sums stay in registers, the row groups meet in
+// shared memory and the CTA writes partials[blockIdx.y, N].
+template <typename T, int ACT, bool WRITE_DZ, bool WANT_SUM, int TX>
 __global__ void __launch_bounds__(256) act_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ z,
                                                       T* __restrict__ dz, float* __restrict__ partials, int M, int N,
                                                       int rows_per_cta) {
-  const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
-  if (c >= N) return;
+  constexpr int TY = 256 / TX;
+  __shared__ float red[WANT_SUM && TY > 1 ? TY : 1][WANT_SUM && TY > 1 ? TX * 8 : 1];
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+  const int c = (blockIdx.x * TX + tx) * 8;
   const int r0 = blockIdx.y * rows_per_cta;
   const int r1 = min(r0 + rows_per_cta, M);
   float acc[8];
@@ -155,62 +161,68 @@ __global__ void __launch_bounds__(256) act_bwd_kernel(const T* __restrict__ dy, 
       for (int i = 0; i < 8; ++i) acc[i] += d[i];
     }
   };
-  int r = r0;
-  for (; r + 1 < r1; r += 2) {
-    const size_t off0 = static_cast<size_t>(r) * N + c, off1 = off0 + N;
-    if (r + 9 < r1) {
-      // the rows this thread reads four iterations from now go to L2 (costs no registers)
-      const size_t offp = off0 + static_cast<size_t>(8) * N;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(dy + offp));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(dy + offp + N));
-      if (ACT != 0) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(z + offp));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(z + offp + N));
+  if (c < N) {
+    int r = r0 + ty;
+    for (; r + TY < r1; r += 2 * TY) {
+      const size_t off0 = static_cast<size_t>(r) * N + c, off1 = off0 + static_cast<size_t>(TY) * N;
+      if (r + 9 * TY < r1) {
+        // the rows this thread reads four iterations from now go to L2 (costs no registers)
+        const size_t offp = off0 + static_cast<size_t>(8 * TY) * N, offq = offp + static_cast<size_t>(TY) * N;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(dy + offp));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(dy + offq));
+        if (ACT != 0) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(z + offp));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(z + offq));
+        }
       }
+      Vec8<T> vd0, vd1, vz0, vz1;
+      vd0.load(dy + off0);
+      vd1.load(dy + off1);
+      if (ACT != 0) {
+        vz0.load(z + off0);
+        vz1.load(z + off1);
+      }
+      one_row(vd0, vz0, off0);
+      one_row(vd1, vz1, off1);
     }
-    Vec8<T> vd0, vd1, vz0, vz1;
-    vd0.load(dy + off0);
-    vd1.load(dy + off1);
-    if (ACT != 0) {
-      vz0.load(z + off0);
-      vz1.load(z + off1);
+    if (r < r1) {
+      const size_t off = static_cast<size_t>(r) * N + c;
+      Vec8<T> vd, vz;
+      vd.load(dy + off);
+      if (ACT != 0) vz.load(z + off);
+      one_row(vd, vz, off);
     }
-    one_row(vd0, vz0, off0);
-    one_row(vd1, vz1, off1);
-  }
-  if (r < r1) {
-    const size_t off = static_cast<size_t>(r) * N + c;
-    Vec8<T> vd, vz;
-    vd.load(dy + off);
-    if (ACT != 0) vz.load(z + off);
-    one_row(vd, vz, off);
   }
   if (WANT_SUM) {
+    if constexpr (TY > 1) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) partials[static_cast<size_t>(blockIdx.y) * N + c + i] = acc[i];
+      for (int i = 0; i < 8; ++i) red[ty][i * TX + tx] = acc[i];      // lanes side by side: no bank conflicts
+      __syncthreads();
+      for (int e = threadIdx.x; e < TX * 8; e += 256) {
+        const int i = e / TX, col = (blockIdx.x * TX + e % TX) * 8 + i;
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < TY; ++q) v += red[q][e];
+        if (col < N) partials[static_cast<size_t>(blockIdx.y) * N + col] = v;
+      }
+    } else if (c < N) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) partials[static_cast<size_t>(blockIdx.y) * N + c + i] = acc[i];
+    }
   }
 }
-
-// out[c] = sum_p part[p, c].  A CTA of 64 columns x 4 row groups: every thread keeps four loads in flight, the row
-// groups meet in shared memory (one thread per column over all P rows left a handful of CTAs waiting on one load each).
-__global__ void __launch_bounds__(256) colsum1_kernel(const float* __restrict__ part, float* __restrict__ out, int P, int N) {
-  __shared__ float red[4][64];
-  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
-  const int c = blockIdx.x * 64 + tx;
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-  if (c < N) {
-    int p = ty;
-    for (; p + 12 < P; p += 16) {
-      a0 += part[static_cast<size_t>(p) * N + c];
-      a1 += part[static_cast<size_t>(p + 4) * N + c];
-      a2 += part[static_cast<size_t>(p + 8) * N + c];
-      a3 += part[static_cast<size_t>(p + 12) * N + c];
-    }
-    for (; p < P; p += 4) a0 += part[static_cast<size_t>(p) * N + c];
+// Threads across the columns of a stripe: the widest of 256, 128, 64, 32 that leaves at most an eighth of them without a
+// column, else the one that leaves fewest.
+static int act_stripe(int N) {
+  const int vecs = N / 8;
+  int best = 256;
+  double best_use = 0.0;
+  for (int tx = 256; tx >= 32; tx /= 2) {
+    const double use = static_cast<double>(vecs) / (static_cast<double>((vecs + tx - 1) / tx) * tx);
+    if (use > best_use + 1e-9) { best = tx; best_use = use; }
+    if (use >= 0.875) break;
   }
-  red[ty][tx] = (a0 + a1) + (a2 + a3);
-  __syncthreads();
-  if (ty == 0 && c < N) out[c] = (red[0][tx] + red[1][tx]) + (red[2][tx] + red[3][tx]);
+  return best;
 }
 
 // ---- embedding -------------------------------------------------------------------------------------------------
@@ -295,40 +307,46 @@ std::vector<torch::Tensor> act_backward(torch::Tensor dy, c10::optional<torch::T
   TORCH_CHECK(N % 8 == 0, "column count must be a multiple of 8");
   if (act != 0) TORCH_CHECK(z.has_value() && z->sizes() == dy.sizes() && z->is_contiguous() && z->dtype() == dy.dtype());
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  const int gx = (N + 2047) / 2048;
-  int gy = std::max(1, std::min((M + 15) / 16, (sms * 8 + gx - 1) / gx));
+  const int tx = act_stripe(std::max(N, 8)), ty = 256 / tx;
+  const int gx = (N + tx * 8 - 1) / (tx * 8);
+  int gy = std::max(1, std::min((M + 8 * ty - 1) / (8 * ty), (sms * 8 + gx - 1) / gx));
   const int rows_per = (M + gy - 1) / gy;
   gy = (M + rows_per - 1) / std::max(rows_per, 1);
   torch::Tensor dz, db, partials;
   if (want_dz) dz = torch::empty_like(dy);
   auto f32 = dy.options().dtype(torch::kFloat32);
   if (want_sum) {
-    partials = torch::empty({std::max(gy, 1), N}, f32);
-    db = torch::zeros({N}, f32);
+    if (M == 0) db = torch::zeros({N}, f32);
+    else db = torch::empty({N}, f32), partials = torch::empty({std::max(gy, 1), N}, f32);
   }
-  if (M == 0) return {dz, db};
+  if (M == 0 || N == 0) return {dz, db};
   auto stream = at::cuda::getCurrentCUDAStream();
   dim3 grid(gx, gy);
 #define LAUNCH_ACT(ACT, WDZ, WSUM)                                                                                  \
-  act_bwd_kernel<T, ACT, WDZ, WSUM><<<grid, 256, 0, stream>>>(                                                      \
+  if (tx == 256) LAUNCH_ACT_TX(ACT, WDZ, WSUM, 256);                                                                \
+  else if (tx == 128) LAUNCH_ACT_TX(ACT, WDZ, WSUM, 128);                                                           \
+  else if (tx == 64) LAUNCH_ACT_TX(ACT, WDZ, WSUM, 64);                                                             \
+  else LAUNCH_ACT_TX(ACT, WDZ, WSUM, 32)
+#define LAUNCH_ACT_TX(ACT, WDZ, WSUM, TX)                                                                           \
+  act_bwd_kernel<T, ACT, WDZ, WSUM, TX><<<grid, 256, 0, stream>>>(                                                    \
       reinterpret_cast<const T*>(dy.data_ptr()), act != 0 ? reinterpret_cast<const T*>(z->data_ptr()) : nullptr,    \
       want_dz ? reinterpret_cast<T*>(dz.data_ptr()) : nullptr, want_sum ? partials.data_ptr<float>() : nullptr, M, N, \
       rows_per)
   DISPATCH_T(dy, {
     if (act == 1) {
-      if (want_sum) LAUNCH_ACT(1, true, true); else LAUNCH_ACT(1, true, false);
+      if (want_sum) { LAUNCH_ACT(1, true, true); } else { LAUNCH_ACT(1, true, false); }
     } else if (act == 2) {
-      if (want_sum) LAUNCH_ACT(2, true, true); else LAUNCH_ACT(2, true, false);
+      if (want_sum) { LAUNCH_ACT(2, true, true); } else { LAUNCH_ACT(2, true, false); }
     } else {
       TORCH_CHECK(!want_dz && want_sum, "identity activation is only used for column sums");
       LAUNCH_ACT(0, false, true);
     }
   })
 #undef LAUNCH_ACT
+#undef LAUNCH_ACT_TX
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   if (want_sum) {
-    colsum1_kernel<<<(N + 63) / 64, 256, 0, stream>>>(partials.data_ptr<float>(), db.data_ptr<float>(), gy, N);
-    C10_CUDA_KERNEL_LAUNCH_CHECK();
+    colsum_launch(partials.data_ptr<float>(), nullptr, db.data_ptr<float>(), nullptr, gy, N, stream);
   }
   return {dz, db};
 }

@@ -17,6 +17,26 @@ def _ops():
     return ops, ext
 
 
+@pytest.mark.parametrize("act", ["gelu", "relu", None])
+@pytest.mark.parametrize("M,N", [(1, 8), (3, 264), (17, 768), (1000, 1600), (513, 3072), (40, 6400), (5000, 2056)])
+def test_act_backward_stripes(M, N, act):
+    ops, _ = _ops()
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    dy = torch.randn(M, N, generator=g, device="cuda").bfloat16()
+    if act is None:
+        got, ref = ops.column_sum(dy), dy.double().sum(0)
+    else:
+        z = torch.randn(M, N, generator=g, device="cuda").bfloat16()
+        zz = z.double().requires_grad_(True)
+        (torch.nn.functional.gelu(zz) if act == "gelu" else zz.relu()).backward(dy.double())
+        dz, got = ops.act_backward(dy, z, act, want_bias_grad=True)
+        # one rounding, and the error function's 1.5e-7 times |dy|
+        assert ((dz.double() - zz.grad).abs() <= UNIT[torch.bfloat16] * zz.grad.abs() + 1e-5).all()
+        ref = dz.double().sum(0)
+    # fp32 sums of M terms below 6 in any order: M * 2^-24 of the sum of the magnitudes
+    assert ((got.double() - ref).abs() <= M * 2.0**-24 * 6 * M + 1e-6).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("trans_a,trans_b", [(False, True), (False, False), (True, False), (True, True)])
 @pytest.mark.parametrize("M,N,K", [
