@@ -10,10 +10,12 @@ choice.
 import contextlib
 
 import torch
+import torch.optim.optimizer as _torch_optimizer
 
+from .optim import FusedAdamW, FusedSGD
 from .parallel.common import synchronize as _sync_async_grads
 from .parallel.ops_1d import PARTIAL_GRAD, reduce_partial_grads
-from .utils.clip_grad import clip_grad_norm
+from .utils.clip_grad import clip_coefficient, clip_grad_norm
 
 
 class Trainer:
@@ -117,13 +119,17 @@ class Trainer:
             reduce_partial_grads(self._partial_params)
         if self.scaler is not None:
             self.scaler.unscale_(self.optimizer)
+        scale = {}
         if self.clip is not None and self.clip > 0:
-            clip_grad_norm(self._params, self.clip)
+            if self._folds_clipping():
+                scale["grad_scale"] = self._clip_factor()
+            else:
+                clip_grad_norm(self._params, self.clip)
         if self.scaler is not None:
             self.scaler.step(self.optimizer)
             self.scaler.update()
         else:
-            self.optimizer.step()
+            self.optimizer.step(**scale)
         if self.lr_scheduler is not None:
             self.lr_scheduler.step()
         self.optimizer.zero_grad(set_to_none=True)
@@ -133,6 +139,26 @@ class Trainer:
         if self.device.type == "cuda" and self.steps % self.status_interval == 0:
             self.check_device_status()
         return total / n if n > 1 else total
+
+    def _folds_clipping(self):
+        """The clipping factor may go into the optimizer's own pass over the gradients: a fused optimizer with its own
+        ``step`` that updates every parameter with a gradient (clipping scales each of them), no loss scaler between, and
+        no hook that could look at the gradients in between."""
+        opt = self.optimizer
+        if self.scaler is not None or type(opt) not in (FusedAdamW, FusedSGD):
+            return False
+        step = opt.__dict__.get("step")              # a learning-rate scheduler wraps it; anything else is the user's
+        if step is not None and not getattr(step, "_wrapped_by_lr_sched", False):
+            return False
+        if opt._optimizer_step_pre_hooks or opt._optimizer_step_post_hooks or \
+                _torch_optimizer._global_optimizer_pre_hooks or _torch_optimizer._global_optimizer_post_hooks:
+            return False
+        covered = {id(p) for group in opt.param_groups for p in group["params"]}
+        return all(id(p) in covered for p in self._params if p.grad is not None)
+
+    def _clip_factor(self):
+        params = [p for p in self._params if p.grad is not None]
+        return clip_coefficient(params, self.clip)[1].float().reshape(1) if params else None
 
     def check_device_status(self):
         """Raise if a kernel of this package gave up on a bounded wait (a peer that never arrived, a stage that

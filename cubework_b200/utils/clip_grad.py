@@ -23,11 +23,21 @@ def _grads(parameters):
 
 
 def clip_grad_norm(parameters, max_norm, norm_type=2):
+    """Scale the gradients in place to a global norm of at most ``max_norm``; returns the norm before."""
     params = _grads(parameters)
-    max_norm = float(max_norm)
-    norm_type = float(norm_type)
     if len(params) == 0:
         return 0.0
+    total_norm, clip_coef = clip_coefficient(params, max_norm, norm_type)
+    from .. import ops
+    ops.scale_grads(params, clip_coef)
+    return total_norm
+
+
+def clip_coefficient(params, max_norm, norm_type=2):
+    """``(global norm, factor)`` as one-element tensors for parameters that have gradients; the gradients are not touched.
+    The fused optimizers take the factor into their update (``grad_scale``), which saves the pass that scales them."""
+    max_norm = float(max_norm)
+    norm_type = float(norm_type)
     tp_on = pm.TENSOR.is_initialized() and pm.TENSOR.world_size > 1
     dp_on = pm.DATA.is_initialized() and pm.DATA.world_size > 1
     device = params[0].grad.device
@@ -67,5 +77,4 @@ def clip_grad_norm(parameters, max_norm, norm_type=2):
             total = total + part
         total_norm = total.pow(1.0 / norm_type)
     clip_coef = (max_norm / (total_norm + 1e-6)).clamp(max=1.0)
-    ops.scale_grads(params, clip_coef)
-    return total_norm.to(device)
+    return total_norm.to(device), clip_coef
