@@ -97,18 +97,19 @@ def masked_embedding(ids, weight, vocab_start=0, out_dtype=None):
 
 
 class _LocalLinear(torch.autograd.Function):
-    """``y = act(x @ op(w) + b)`` on this rank only; ``w_is_out_in`` selects ``[out,in]`` vs ``[in,out]``."""
+    """``y = act(x @ op(w) + b)`` on this rank only; ``w_is_out_in`` selects ``[out,in]`` vs ``[in,out]``.  The
+    pre-activation copy is only written when a backward pass can follow (``keep_z``)."""
 
     @staticmethod
-    def forward(ctx, x, w, b, w_is_out_in, act):
+    def forward(ctx, x, w, b, w_is_out_in, act, keep_z):
         cd = ops.compute_dtype(x)
         x2 = as_compute(x.reshape(-1, x.shape[-1]), cd)
         wc = ops.shadow(w, cd)
         z = None
-        if act is not None:
+        if act is not None and keep_z:
             y, z = ops.gemm(x2, wc, trans_b=w_is_out_in, bias=b, act=act, pre_act_out=True)
         else:
-            y = ops.gemm(x2, wc, trans_b=w_is_out_in, bias=b)
+            y = ops.gemm(x2, wc, trans_b=w_is_out_in, bias=b, act=act)
         ctx.save_for_backward(x2, w, z if z is not None else x2.new_empty(0))
         ctx.cfg = (cd, w_is_out_in, act, b is not None, b.dtype if b is not None else None, x.dtype, x.shape)
         return y.view(*x.shape[:-1], y.shape[-1])
@@ -135,8 +136,8 @@ class _LocalLinear(torch.autograd.Function):
                 dw = ops.gemm(dy2, x2, trans_a=True, out_dtype=w.dtype)
             else:
                 dw = ops.gemm(x2, dy2, trans_a=True, out_dtype=w.dtype)
-        return dx, dw, db, None, None
+        return dx, dw, db, None, None, None
 
 
 def local_linear(x, w, b=None, w_is_out_in=True, act=None):
-    return _LocalLinear.apply(x, w, b, w_is_out_in, act)
+    return _LocalLinear.apply(x, w, b, w_is_out_in, act, torch.is_grad_enabled())

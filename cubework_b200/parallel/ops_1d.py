@@ -119,10 +119,11 @@ class _Linear1D(torch.autograd.Function):
 
     ``reduce_fwd``: sum ``y`` over the group (row-parallel; bias added once, after the sum).
     ``reduce_bwd``: sum ``dx`` over the group (column-parallel, replicated input).
+    ``keep_z``: a backward pass can follow, so the activation's input is written as well.
     """
 
     @staticmethod
-    def forward(ctx, x, w, b, mode, reduce_fwd, reduce_bwd, act, skip=False):
+    def forward(ctx, x, w, b, mode, reduce_fwd, reduce_bwd, act, skip=False, keep_z=True):
         cd = ops.compute_dtype(x)
         x2 = x.reshape(-1, x.shape[-1])
         if x2.dtype != cd:
@@ -136,10 +137,10 @@ class _Linear1D(torch.autograd.Function):
         elif reduce_fwd and mode.world_size > 1:
             assert act is None
             y = fused.gemm_all_reduce(x2, wc, False, True, mode, bias=b)
-        elif act is not None:
+        elif act is not None and keep_z:
             y, z = ops.gemm(x2, wc, trans_b=True, bias=b, act=act, pre_act_out=True)
         else:
-            y = ops.gemm(x2, wc, trans_b=True, bias=b)
+            y = ops.gemm(x2, wc, trans_b=True, bias=b, act=act)
         ctx.save_for_backward(x2, w, z if z is not None else x2.new_empty(0))
         ctx.mode, ctx.reduce_bwd, ctx.act, ctx.cd = mode, reduce_bwd, act, cd
         ctx.has_bias = b is not None
@@ -180,11 +181,11 @@ class _Linear1D(torch.autograd.Function):
             dx = dx.view(ctx.x_shape)
             if dx.dtype != ctx.x_dtype:
                 dx = dx.to(ctx.x_dtype)
-        return dx, dw, db, None, None, None, None, None
+        return dx, dw, db, None, None, None, None, None, None
 
 
 def linear_1d(x, w, b, mode, reduce_fwd=False, reduce_bwd=False, act=None, skip=False):
-    return _Linear1D.apply(x, w, b, mode, reduce_fwd, reduce_bwd, act, skip)
+    return _Linear1D.apply(x, w, b, mode, reduce_fwd, reduce_bwd, act, skip, torch.is_grad_enabled())
 
 
 class _Linear1DRows(torch.autograd.Function):
@@ -280,7 +281,7 @@ class _Linear1DRows(torch.autograd.Function):
 def linear_1d_rows(x, w, b, mode, kind, act=None, skip=False):
     """See :class:`_Linear1DRows`; with a group of one this is the plain linear."""
     if mode.world_size == 1:
-        return _Linear1D.apply(x, w, b, mode, False, False, act, skip)
+        return _Linear1D.apply(x, w, b, mode, False, False, act, skip, torch.is_grad_enabled())
     return _Linear1DRows.apply(x, w, b, mode, kind, act, skip)
 
 
