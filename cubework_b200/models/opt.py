@@ -86,30 +86,35 @@ class OPTDecoderLayer(nn.Module):
     fc1 = property(lambda self: self.ffn.dense_1)
     fc2 = property(lambda self: self.ffn.dense_2)
 
-    def _forward(self, h, key_bias=None, past_key_value=None, use_cache=False):
-        residual = h
-        if self.do_layer_norm_before:
-            h = self.self_attn_layer_norm(h)
-        present = None
+    def _attend(self, h, key_bias, past_key_value, use_cache):
         if use_cache or past_key_value is not None:
-            h, present = self.self_attn.forward_cached(h, past_key_value, key_bias)
-        else:
-            h = self.self_attn(h, key_bias)
-        h = residual + self.dropout(h)
-        if not self.do_layer_norm_before:
-            h = self.self_attn_layer_norm(h)
-        residual = h
-        if self.do_layer_norm_before:
-            h = self.final_layer_norm(h)
-        h = residual + self.ffn(h)
-        if not self.do_layer_norm_before:
-            h = self.final_layer_norm(h)
-        return h, present
+            return self.self_attn.forward_cached(h, past_key_value, key_bias)
+        return self.self_attn(h, key_bias), None
 
-    def forward(self, h, key_bias=None, past_key_value=None, use_cache=False):
+    def _forward(self, h, key_bias=None, past_key_value=None, use_cache=False, pending=None, defer=False):
+        if not self.do_layer_norm_before:
+            a, present = self._attend(h, key_bias, past_key_value, use_cache)
+            h = self.self_attn_layer_norm(h + self.dropout(a))
+            return self.final_layer_norm(h + self.ffn(h)), present
+        if pending is None:
+            n = self.self_attn_layer_norm(h)
+        else:
+            h, n = self.self_attn_layer_norm(h, residual=pending)
+        a, present = self._attend(n, key_bias, past_key_value, use_cache)
+        h, n = self.final_layer_norm(h, residual=self.dropout(a))
+        out = self.ffn(n)
+        return (h, out, present) if defer else (h + out, present)
+
+    def forward(self, h, key_bias=None, past_key_value=None, use_cache=False, pending=None, defer=False):
+        """``(h, present)``.  A pre-LN layer with ``defer`` leaves its last residual add to the norm that follows and
+        returns ``(stream, contribution, present)``; ``pending`` is such a contribution of the layer before (the norms
+        compute the sum and its normalised value in one kernel)."""
         if self.gradient_checkpointing and self.training and not use_cache:
+            if defer:
+                out = maybe_checkpoint(lambda a, c, b: self._forward(a, b, pending=c, defer=True)[:2], True, h, pending, key_bias)
+                return (*out, None)
             return maybe_checkpoint(lambda a, b: self._forward(a, b)[0], True, h, key_bias), None
-        return self._forward(h, key_bias, past_key_value, use_cache)
+        return self._forward(h, key_bias, past_key_value, use_cache, pending, defer)
 
 
 class OPTLMLoss(nn.Module):
@@ -164,14 +169,20 @@ class OPT(nn.Module):
             key_bias = key_bias_from_mask(attention_mask)
         h = h + self.embed_positions(mask_full, past_len)
         cache = () if use_cache else None
+        defer, pending = self.final_layer_norm is not None, None
         for idx, layer in enumerate(self.layers):
             if self.training and self.layerdrop > 0 and torch.rand(()).item() < self.layerdrop:
                 continue
             past = past_key_values[idx] if past_key_values is not None else None
-            h, present = layer(h, key_bias, past, use_cache)
+            if defer:
+                h, pending, present = layer(h, key_bias, past, use_cache, pending, True)
+            else:
+                h, present = layer(h, key_bias, past, use_cache)
             if use_cache:
                 cache += (present, )
-        if self.final_layer_norm is not None:
+        if pending is not None:
+            h = self.final_layer_norm(h, residual=pending)[1]
+        elif defer:
             h = self.final_layer_norm(h)
         logits = self.lm_head(h)
         return (logits, cache) if use_cache else (logits, )

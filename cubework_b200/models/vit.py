@@ -64,12 +64,19 @@ class ViTBlock(nn.Module):
                        inner_dropout=dropout)
         mark_block_output(self.mlp.dense_2)
 
-    def _forward(self, x):
-        x = x + self.drop_path(self.attn(self.norm1(x)))
-        return x + self.drop_path(self.mlp(self.norm2(x)))
+    def _forward(self, x, pending=None, defer=False):
+        if pending is None:
+            n = self.norm1(x)
+        else:
+            x, n = self.norm1(x, residual=pending)
+        x, n = self.norm2(x, residual=self.drop_path(self.attn(n)))
+        out = self.drop_path(self.mlp(n))
+        return (x, out) if defer else x + out
 
-    def forward(self, x):
-        return maybe_checkpoint(self._forward, self.checkpoint, x)
+    def forward(self, x, pending=None, defer=False):
+        """The block's output; with ``defer`` its last residual add is left to the norm that follows and
+        ``(stream, contribution)`` is returned.  ``pending`` is such a contribution of the block before."""
+        return maybe_checkpoint(self._forward, self.checkpoint, x, pending, defer)
 
 
 class VisionTransformer(nn.Module):
@@ -92,9 +99,10 @@ class VisionTransformer(nn.Module):
 
     def forward(self, pixel_values):
         x = self.embed(pixel_values)
+        pending = None
         for block in self.blocks:
-            x = block(x)
-        return self.head(self.norm(x))
+            x, pending = block(x, pending, True)
+        return self.head(self.norm(x) if pending is None else self.norm(x, residual=pending)[1])
 
 
 class MixupLoss(nn.Module):

@@ -10,12 +10,13 @@
 #include <c10/cuda/CUDAException.h>
 #include <torch/extension.h>
 
+#include "colsum.cuh"
 #include "common.cuh"
 
 namespace cw {
 
 constexpr int kNT = 256;
-constexpr int kMaxVPT = 8;   // 8 vectors x 8 elements x 256 threads = 16384 columns; kernels are compiled for 1, 2, 4, 8
+constexpr int kMaxVPT = 8;   // 8 vectors x 8 elements x 256 threads = 16384 columns; kernels are compiled for 1, 2, 3, 4, 8
 
 template <typename T, int VPT>
 __device__ __forceinline__ int load_row(const T* row, int H, float (&x)[VPT][8]) {
@@ -36,32 +37,107 @@ __device__ __forceinline__ int load_row(const T* row, int H, float (&x)[VPT][8])
   return n;
 }
 
-// MODE 0: local statistics (plain layer norm).  MODE 1: statistics supplied (sharded, pass 2).
-template <typename T, int MODE, int VPT>
-__global__ void __launch_bounds__(kNT) ln_fwd_kernel(const T* __restrict__ x, const float* __restrict__ gamma,
-                                                     const float* __restrict__ beta, T* __restrict__ y,
+// 8 consecutive norm parameters as two 16-byte loads (as eight scalar loads, 32 bytes apart between lanes, they kept the
+// L1 busier than the rows did: 118 us for 8192 x 5120, which is 168 MB).
+__device__ __forceinline__ void load8f(const float* p, float (&f)[8]) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+template <typename T>
+__device__ __forceinline__ void unpack8(const uint4& raw, float (&f)[8]) {
+  const T* h = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) f[i] = to_f(h[i]);
+}
+template <typename T>
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  uint4 raw;
+  T* h = reinterpret_cast<T*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) h[i] = from_f<T>(f[i]);
+  return raw;
+}
+
+__device__ __forceinline__ void load8p(const float* p, float (&f)[8]) { load8f(p, f); }
+template <typename T>
+__device__ __forceinline__ void load8p(const T* p, float (&f)[8]) { unpack8<T>(__ldg(reinterpret_cast<const uint4*>(p)), f); }
+
+// P below: type of the norm parameters, fp32 or that of the rows (models that keep their parameters in 16 bits; converting
+// them took two launches per call, as long as the norm of a few rows itself).
+//
+// MODE 0: local statistics (plain layer norm), optionally of x + res, which is written out as well (HAS_RES).
+// MODE 1: statistics supplied (sharded, pass 2).  The row stays in registers as it was loaded (16 bits); the next row
+// of the CTA is requested into L2 meanwhile.  8192 x 5120: 118 -> 60 us (168 MB), 73 with the residual (336 MB, which took
+// an add of 39 us and a norm of 118).
+template <typename T, int MODE, int VPT, bool HAS_RES, typename P>
+__global__ void __launch_bounds__(kNT) ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ res,
+                                                     const P* __restrict__ gamma, const P* __restrict__ beta,
+                                                     T* __restrict__ sum_out, T* __restrict__ y,
                                                      float* __restrict__ mean_io, float* __restrict__ rstd_io, int rows,
                                                      int H, float eps) {
   __shared__ float red[64];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    float xv[VPT][8];
-    load_row(x + static_cast<size_t>(row) * H, H, xv);
+    const size_t base = static_cast<size_t>(row) * H;
+    uint4 raw[VPT], rr[HAS_RES ? VPT : 1];
+#pragma unroll
+    for (int v = 0; v < VPT; ++v) {
+      const int c = (v * kNT + threadIdx.x) * 8;
+      raw[v] = c < H ? *reinterpret_cast<const uint4*>(x + base + c) : make_uint4(0, 0, 0, 0);
+      if (HAS_RES) rr[v] = c < H ? *reinterpret_cast<const uint4*>(res + base + c) : make_uint4(0, 0, 0, 0);
+    }
+    // a row that fills the threads once: its parameters are requested with it, not after the two reductions
+    float g0[8], be0[8];
+    if constexpr (VPT == 1) {
+      if (gamma != nullptr && static_cast<int>(threadIdx.x) * 8 < H) {
+        load8p(gamma + threadIdx.x * 8, g0);
+        load8p(beta + threadIdx.x * 8, be0);
+      }
+    }
+    if (row + gridDim.x < rows) {
+      const size_t nbase = base + static_cast<size_t>(gridDim.x) * H;
+#pragma unroll
+      for (int v = 0; v < VPT; ++v) {
+        const int c = (v * kNT + threadIdx.x) * 8;
+        if (c < H) {
+          prefetch_l2(x + nbase + c);
+          if (HAS_RES) prefetch_l2(res + nbase + c);
+        }
+      }
+    }
+    if (HAS_RES) {
+#pragma unroll
+      for (int v = 0; v < VPT; ++v) {
+        const int c = (v * kNT + threadIdx.x) * 8;
+        float a[8], b[8];
+        unpack8<T>(raw[v], a);
+        unpack8<T>(rr[v], b);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] += b[i];
+        raw[v] = pack8<T>(a);                         // the normalised value is that of the stored (rounded) sum
+        if (c < H) *reinterpret_cast<uint4*>(sum_out + base + c) = raw[v];
+      }
+    }
     float mean, rstd;
     if (MODE == 0) {
       float s = 0.f, dummy = 0.f;
 #pragma unroll
-      for (int v = 0; v < VPT; ++v)
+      for (int v = 0; v < VPT; ++v) {
+        float f[8];
+        unpack8<T>(raw[v], f);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s += xv[v][i];
+        for (int i = 0; i < 8; ++i) s += f[i];
+      }
       block_sum2<kNT>(s, dummy, red);
       mean = s / H;
       float q = 0.f;
 #pragma unroll
       for (int v = 0; v < VPT; ++v) {
-        const int c = (v * kNT + threadIdx.x) * 8;
-        if (c < H) {
+        if ((v * kNT + threadIdx.x) * 8 < H) {
+          float f[8];
+          unpack8<T>(raw[v], f);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) { const float d = xv[v][i] - mean; q += d * d; }
+          for (int i = 0; i < 8; ++i) { const float d = f[i] - mean; q += d * d; }
         }
       }
       block_sum2<kNT>(q, dummy, red);
@@ -75,16 +151,20 @@ __global__ void __launch_bounds__(kNT) ln_fwd_kernel(const T* __restrict__ x, co
     for (int v = 0; v < VPT; ++v) {
       const int c = (v * kNT + threadIdx.x) * 8;
       if (c < H) {
-        float o[8];
+        float f[8];
+        unpack8<T>(raw[v], f);
+        if (gamma != nullptr) {
+          if constexpr (VPT > 1) {
+            load8p(gamma + c, g0);
+            load8p(beta + c, be0);
+          }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float n = (xv[v][i] - mean) * rstd;
-          if (gamma != nullptr) n = n * __ldg(gamma + c + i) + __ldg(beta + c + i);
-          o[i] = n;
+          for (int i = 0; i < 8; ++i) f[i] = (f[i] - mean) * rstd * g0[i] + be0[i];
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) f[i] = (f[i] - mean) * rstd;
         }
-        Vec8<T> t;
-        t.pack(o);
-        t.store(y + static_cast<size_t>(row) * H + c);
+        *reinterpret_cast<uint4*>(y + base + c) = pack8<T>(f);
       }
     }
   }
@@ -108,14 +188,18 @@ __global__ void __launch_bounds__(kNT) row_moments_kernel(const T* __restrict__ 
   }
 }
 
-// Backward.  MODE 0: everything local.  MODE 1: only row sums [sum g, sum g*xhat] + parameter partials.
-// MODE 2: only dx, row sums supplied (already reduced over the group) and divided by `hidden`.
-template <typename T, int MODE, int VPT>
-__global__ void __launch_bounds__(kNT) ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
+// Backward.  MODE 0: everything local, optionally plus the gradient that reaches the normalised tensor directly
+// (HAS_RES).  MODE 1: only row sums [sum g, sum g*xhat] + parameter partials.  MODE 2: only dx, row sums supplied
+// (already reduced over the group) and divided by `hidden`.  Rows stay in registers as they were loaded (16 bits) and
+// are converted twice; the next row is requested into L2 meanwhile.  8192 x 5120: 181 -> 83 us, 117 with the residual's
+// gradient (336 MB; 205 while it was left at one CTA per SM by its registers).
+template <typename T, int MODE, int VPT, bool HAS_RES>
+__global__ void __launch_bounds__(kNT, VPT <= 3 ? 2 : 1) ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                                                      const float* __restrict__ mean, const float* __restrict__ rstd,
-                                                     const float* __restrict__ gamma, T* __restrict__ dx,
-                                                     float* __restrict__ row_sums, float* __restrict__ part_dgamma,
-                                                     float* __restrict__ part_dbeta, int rows, int H, float hidden) {
+                                                     const float* __restrict__ gamma, const T* __restrict__ dres,
+                                                     T* __restrict__ dx, float* __restrict__ row_sums,
+                                                     float* __restrict__ part_dgamma, float* __restrict__ part_dbeta,
+                                                     int rows, int H, float hidden) {
   __shared__ float red[64];
   float dg[VPT][8], db[VPT][8];
 #pragma unroll
@@ -124,34 +208,56 @@ __global__ void __launch_bounds__(kNT) ln_bwd_kernel(const T* __restrict__ dy, c
     for (int i = 0; i < 8; ++i) { dg[v][i] = 0.f; db[v][i] = 0.f; }
 
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    float xv[VPT][8], gv[VPT][8];
-    load_row(x + static_cast<size_t>(row) * H, H, xv);
-    load_row(dy + static_cast<size_t>(row) * H, H, gv);
-    const float mu = mean[row], rs = rstd[row];
-    float s1 = 0.f, s2 = 0.f;
+    const size_t base = static_cast<size_t>(row) * H;
+    uint4 xr[VPT], gr[VPT];
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
       const int c = (v * kNT + threadIdx.x) * 8;
-      if (c < H) {
+      xr[v] = c < H ? *reinterpret_cast<const uint4*>(x + base + c) : make_uint4(0, 0, 0, 0);
+      gr[v] = c < H ? *reinterpret_cast<const uint4*>(dy + base + c) : make_uint4(0, 0, 0, 0);
+    }
+    {
+      const size_t nbase = base + static_cast<size_t>(gridDim.x) * H;
+      const bool has_next = row + gridDim.x < rows;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float xhat = (xv[v][i] - mu) * rs;
-          const float d = gv[v][i];
-          if (MODE != 2) { dg[v][i] += d * xhat; db[v][i] += d; }
-          const float g = gamma != nullptr ? d * __ldg(gamma + c + i) : d;
-          xv[v][i] = xhat;
-          gv[v][i] = g;
-          s1 += g;
-          s2 += g * xhat;
+      for (int v = 0; v < VPT; ++v) {
+        const int c = (v * kNT + threadIdx.x) * 8;
+        if (c < H) {
+          if (HAS_RES) prefetch_l2(dres + base + c);
+          if (has_next) {
+            prefetch_l2(x + nbase + c);
+            prefetch_l2(dy + nbase + c);
+          }
         }
       }
     }
-    if (MODE == 2) {
-      s1 = row_sums[2 * row];
-      s2 = row_sums[2 * row + 1];
-    } else {
+    const float mu = mean[row], rs = rstd[row];
+    float s1 = 0.f, s2 = 0.f;
+    if (MODE != 2) {
+#pragma unroll
+      for (int v = 0; v < VPT; ++v) {
+        const int c = (v * kNT + threadIdx.x) * 8;
+        if (c < H) {
+          float xf[8], gf[8], gm[8];
+          unpack8<T>(xr[v], xf);
+          unpack8<T>(gr[v], gf);
+          if (gamma != nullptr) load8f(gamma + c, gm);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float xhat = (xf[i] - mu) * rs;
+            dg[v][i] += gf[i] * xhat;
+            db[v][i] += gf[i];
+            const float g = gamma != nullptr ? gf[i] * gm[i] : gf[i];
+            s1 += g;
+            s2 += g * xhat;
+          }
+        }
+      }
       block_sum2<kNT>(s1, s2, red);
       if (MODE == 1 && threadIdx.x == 0) { row_sums[2 * row] = s1; row_sums[2 * row + 1] = s2; }
+    } else {
+      s1 = row_sums[2 * row];
+      s2 = row_sums[2 * row + 1];
     }
     if (MODE != 1) {
       const float m1 = s1 / hidden, m2 = s2 / hidden;
@@ -159,12 +265,19 @@ __global__ void __launch_bounds__(kNT) ln_bwd_kernel(const T* __restrict__ dy, c
       for (int v = 0; v < VPT; ++v) {
         const int c = (v * kNT + threadIdx.x) * 8;
         if (c < H) {
-          float o[8];
+          float xf[8], gf[8], gm[8], rv[8];
+          unpack8<T>(xr[v], xf);
+          unpack8<T>(gr[v], gf);
+          if (gamma != nullptr) load8f(gamma + c, gm);
+          if (HAS_RES) unpack8<T>(*reinterpret_cast<const uint4*>(dres + base + c), rv);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = (gv[v][i] - m1 - xv[v][i] * m2) * rs;
-          Vec8<T> t;
-          t.pack(o);
-          t.store(dx + static_cast<size_t>(row) * H + c);
+          for (int i = 0; i < 8; ++i) {
+            const float xhat = (xf[i] - mu) * rs;
+            const float g = gamma != nullptr ? gf[i] * gm[i] : gf[i];
+            xf[i] = (g - m1 - xhat * m2) * rs;
+            if (HAS_RES) xf[i] += rv[i];
+          }
+          *reinterpret_cast<uint4*>(dx + base + c) = pack8<T>(xf);
         }
       }
     }
@@ -174,11 +287,12 @@ __global__ void __launch_bounds__(kNT) ln_bwd_kernel(const T* __restrict__ dy, c
     for (int v = 0; v < VPT; ++v) {
       const int c = (v * kNT + threadIdx.x) * 8;
       if (c < H) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          part_dgamma[static_cast<size_t>(blockIdx.x) * H + c + i] = dg[v][i];
-          part_dbeta[static_cast<size_t>(blockIdx.x) * H + c + i] = db[v][i];
-        }
+        float4* pg = reinterpret_cast<float4*>(part_dgamma + static_cast<size_t>(blockIdx.x) * H + c);
+        float4* pb = reinterpret_cast<float4*>(part_dbeta + static_cast<size_t>(blockIdx.x) * H + c);
+        pg[0] = make_float4(dg[v][0], dg[v][1], dg[v][2], dg[v][3]);
+        pg[1] = make_float4(dg[v][4], dg[v][5], dg[v][6], dg[v][7]);
+        pb[0] = make_float4(db[v][0], db[v][1], db[v][2], db[v][3]);
+        pb[1] = make_float4(db[v][4], db[v][5], db[v][6], db[v][7]);
       }
     }
   }
@@ -192,25 +306,10 @@ __global__ void __launch_bounds__(kNT) ln_bwd_kernel(const T* __restrict__ dy, c
 // and its normalised value, backward adds the gradient that reaches the sum directly.
 constexpr int kWarpRows = 8;                 // warps (rows in flight) per CTA
 
-template <typename T>
-__device__ __forceinline__ void unpack8(const uint4& raw, float (&f)[8]) {
-  const T* h = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) f[i] = to_f(h[i]);
-}
-template <typename T>
-__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
-  uint4 raw;
-  T* h = reinterpret_cast<T*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) h[i] = from_f<T>(f[i]);
-  return raw;
-}
-
-template <typename T, int NV, bool HAS_RES>
+template <typename T, int NV, bool HAS_RES, typename P>
 __global__ void __launch_bounds__(32 * kWarpRows)
-ln_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res, const float* __restrict__ gamma,
-                   const float* __restrict__ beta, T* __restrict__ sum_out, T* __restrict__ y, float* __restrict__ mean_o,
+ln_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res, const P* __restrict__ gamma,
+                   const P* __restrict__ beta, T* __restrict__ sum_out, T* __restrict__ y, float* __restrict__ mean_o,
                    float* __restrict__ rstd_o, int rows, int H, float eps) {
   const int lane = threadIdx.x & 31;
   const int warp = blockIdx.x * kWarpRows + (threadIdx.x >> 5);
@@ -279,10 +378,9 @@ ln_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res, const flo
       if (c < H) {
         float f[8];
         unpack8<T>(raw[v], f);
-        const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + c)), g1 = __ldg(reinterpret_cast<const float4*>(gamma + c + 4));
-        const float4 b0 = __ldg(reinterpret_cast<const float4*>(beta + c)), b1 = __ldg(reinterpret_cast<const float4*>(beta + c + 4));
-        const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-        const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+        float gg[8], bb[8];
+        load8p(gamma + c, gg);
+        load8p(beta + c, bb);
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] = (f[i] - mean) * rstd * gg[i] + bb[i];
         *reinterpret_cast<uint4*>(y + base + c) = pack8<T>(f);
@@ -294,7 +392,7 @@ ln_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res, const flo
 // Backward of the above.  Each warp keeps the dgamma / dbeta partial sums of its rows in a shared-memory strip of its
 // own (in registers they cost 112 registers per thread at H = 1600 and held the kernel at eight warps per SM, where it
 // was bound by latency); the warps of a CTA are added up at the end and the CTA writes one partial row (summed by
-// colsum2).
+// colsum_kernel).
 template <typename T, int NV, bool HAS_RES>
 __global__ void __launch_bounds__(32 * kWarpRows, 2)
 ln_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ mean,
@@ -420,20 +518,6 @@ static void launch_ln_bwd_warp(int grid, size_t smem, cudaStream_t stream, const
                                                reinterpret_cast<const T*>(dres), reinterpret_cast<T*>(dx), pdg, pdb, rows, H);
 }
 
-// out[c] = sum_p part[p, c] for two partial buffers at once.
-__global__ void colsum2_kernel(const float* __restrict__ pa, const float* __restrict__ pb, float* __restrict__ oa,
-                               float* __restrict__ ob, int P, int H) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= H) return;
-  float a = 0.f, b = 0.f;
-  for (int p = 0; p < P; ++p) {
-    a += pa[static_cast<size_t>(p) * H + c];
-    b += pb[static_cast<size_t>(p) * H + c];
-  }
-  oa[c] = a;
-  ob[c] = b;
-}
-
 // ---------------------------------------------------------------------------------------- host side
 static void check_rows(const torch::Tensor& x) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.is_contiguous(), "expected a contiguous 2-D CUDA tensor");
@@ -455,6 +539,7 @@ static const float* fptr(const c10::optional<torch::Tensor>& t) {
     const int need_ = ((H) / 8 + kNT - 1) / kNT;                    \
     if (need_ <= 1) { constexpr int VPT = 1; __VA_ARGS__ }          \
     else if (need_ <= 2) { constexpr int VPT = 2; __VA_ARGS__ }     \
+    else if (need_ <= 3) { constexpr int VPT = 3; __VA_ARGS__ }     \
     else if (need_ <= 4) { constexpr int VPT = 4; __VA_ARGS__ }     \
     else { constexpr int VPT = 8; __VA_ARGS__ }                     \
   }
@@ -467,19 +552,50 @@ static const float* fptr(const c10::optional<torch::Tensor>& t) {
     DISPATCH_VPT((x).size(1), __VA_ARGS__)                          \
   }
 
-std::vector<torch::Tensor> layer_norm_fwd(torch::Tensor x, torch::Tensor gamma, torch::Tensor beta, double eps) {
+// The kernels read norm parameters in 16-byte pieces; a view that starts elsewhere (a slice of a flat buffer) is copied.
+static torch::Tensor aligned16(const torch::Tensor& t) {
+  return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone();
+}
+static c10::optional<torch::Tensor> aligned16(const c10::optional<torch::Tensor>& t) {
+  if (!t.has_value() || !t->defined()) return t;
+  return aligned16(*t);
+}
+
+static std::vector<torch::Tensor> layer_norm_fwd_cta(torch::Tensor x, const torch::Tensor* res, torch::Tensor gamma,
+                                                     torch::Tensor beta, double eps) {
   check_rows(x);
   const int rows = x.size(0), H = x.size(1);
+  gamma = aligned16(gamma);
+  beta = aligned16(beta);
   auto y = torch::empty_like(x);
   auto mean = torch::empty({rows}, x.options().dtype(torch::kFloat32));
   auto rstd = torch::empty({rows}, x.options().dtype(torch::kFloat32));
-  if (rows == 0) return {y, mean, rstd};
+  torch::Tensor sum;
+  if (res != nullptr) sum = torch::empty_like(x);
+  if (rows == 0) return {y, mean, rstd, sum};
   auto stream = at::cuda::getCurrentCUDAStream();
-  DISPATCH_16(x, ln_fwd_kernel<T, 0, VPT><<<row_grid(rows), kNT, 0, stream>>>(
-                     reinterpret_cast<const T*>(x.data_ptr()), fptr(gamma), fptr(beta), reinterpret_cast<T*>(y.data_ptr()),
-                     mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, H, static_cast<float>(eps));)
+#define LAUNCH_LN_CTA(RES, P)                                                                                             \
+  ln_fwd_kernel<T, 0, VPT, RES, P><<<row_grid(rows), kNT, 0, stream>>>(                                                   \
+      reinterpret_cast<const T*>(x.data_ptr()), RES ? reinterpret_cast<const T*>(res->data_ptr()) : nullptr,              \
+      reinterpret_cast<const P*>(gamma.data_ptr()), reinterpret_cast<const P*>(beta.data_ptr()),                          \
+      RES ? reinterpret_cast<T*>(sum.data_ptr()) : nullptr, reinterpret_cast<T*>(y.data_ptr()), mean.data_ptr<float>(),   \
+      rstd.data_ptr<float>(), rows, H, static_cast<float>(eps))
+  const bool f32 = gamma.scalar_type() == torch::kFloat32;
+  DISPATCH_16(x, {
+    if (res != nullptr) { if (f32) LAUNCH_LN_CTA(true, float); else LAUNCH_LN_CTA(true, T); }
+    else { if (f32) LAUNCH_LN_CTA(false, float); else LAUNCH_LN_CTA(false, T); }
+  })
+#undef LAUNCH_LN_CTA
   C10_CUDA_KERNEL_LAUNCH_CHECK();
-  return {y, mean, rstd};
+  return {y, mean, rstd, sum};
+}
+
+std::vector<torch::Tensor> layer_norm_fwd(torch::Tensor x, torch::Tensor gamma, torch::Tensor beta, double eps) {
+  TORCH_CHECK(gamma.scalar_type() == torch::kFloat32 && beta.scalar_type() == torch::kFloat32 && gamma.is_contiguous() &&
+              beta.is_contiguous(), "norm parameters must be contiguous fp32");
+  auto r = layer_norm_fwd_cta(x, nullptr, gamma, beta, eps);
+  r.pop_back();
+  return r;
 }
 
 torch::Tensor norm_apply(torch::Tensor x, torch::Tensor mean, torch::Tensor rstd, c10::optional<torch::Tensor> gamma,
@@ -489,9 +605,11 @@ torch::Tensor norm_apply(torch::Tensor x, torch::Tensor mean, torch::Tensor rstd
   auto y = torch::empty_like(x);
   if (rows == 0) return y;
   auto stream = at::cuda::getCurrentCUDAStream();
-  DISPATCH_16(x, ln_fwd_kernel<T, 1, VPT><<<row_grid(rows), kNT, 0, stream>>>(
-                     reinterpret_cast<const T*>(x.data_ptr()), fptr(gamma), fptr(beta), reinterpret_cast<T*>(y.data_ptr()),
-                     mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, H, 0.f);)
+  gamma = aligned16(gamma);
+  beta = aligned16(beta);
+  DISPATCH_16(x, ln_fwd_kernel<T, 1, VPT, false, float><<<row_grid(rows), kNT, 0, stream>>>(
+                     reinterpret_cast<const T*>(x.data_ptr()), nullptr, fptr(gamma), fptr(beta), nullptr,
+                     reinterpret_cast<T*>(y.data_ptr()), mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, H, 0.f);)
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   return y;
 }
@@ -511,12 +629,18 @@ torch::Tensor row_moments(torch::Tensor x) {
 // Launches the backward kernel on caller-provided scratch: part_dgamma / part_dbeta are [grid, H] fp32.
 template <int MODE>
 static void ln_bwd_launch(const torch::Tensor& dy, const torch::Tensor& x, const float* mean, const float* rstd,
-                          const float* gamma, void* dx, float* row_sums, float* pdg, float* pdb, int grid, float hidden,
-                          cudaStream_t stream) {
+                          const float* gamma, const void* dres, void* dx, float* row_sums, float* pdg, float* pdb, int grid,
+                          float hidden, cudaStream_t stream) {
   const int rows = x.size(0), H = x.size(1);
-  DISPATCH_16(x, ln_bwd_kernel<T, MODE, VPT><<<grid, kNT, 0, stream>>>(
-                     reinterpret_cast<const T*>(dy.data_ptr()), reinterpret_cast<const T*>(x.data_ptr()), mean, rstd, gamma,
-                     reinterpret_cast<T*>(dx), row_sums, pdg, pdb, rows, H, hidden);)
+  if (MODE == 0 && dres != nullptr) {
+    DISPATCH_16(x, ln_bwd_kernel<T, 0, VPT, true><<<grid, kNT, 0, stream>>>(
+                       reinterpret_cast<const T*>(dy.data_ptr()), reinterpret_cast<const T*>(x.data_ptr()), mean, rstd, gamma,
+                       reinterpret_cast<const T*>(dres), reinterpret_cast<T*>(dx), row_sums, pdg, pdb, rows, H, hidden);)
+  } else {
+    DISPATCH_16(x, ln_bwd_kernel<T, MODE, VPT, false><<<grid, kNT, 0, stream>>>(
+                       reinterpret_cast<const T*>(dy.data_ptr()), reinterpret_cast<const T*>(x.data_ptr()), mean, rstd, gamma,
+                       nullptr, reinterpret_cast<T*>(dx), row_sums, pdg, pdb, rows, H, hidden);)
+  }
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 
@@ -525,25 +649,31 @@ static int bwd_grid(int rows) {
   return std::max(1, std::min(rows, sms * 2));
 }
 
-std::vector<torch::Tensor> layer_norm_bwd(torch::Tensor dy, torch::Tensor x, torch::Tensor mean, torch::Tensor rstd,
-                                          torch::Tensor gamma) {
+static std::vector<torch::Tensor> layer_norm_bwd_cta(torch::Tensor dy, torch::Tensor x, torch::Tensor mean, torch::Tensor rstd,
+                                                     torch::Tensor gamma, const torch::Tensor* dres) {
   check_rows(x);
   check_rows(dy);
   const int rows = x.size(0), H = x.size(1);
+  gamma = aligned16(gamma);
   auto dx = torch::empty_like(x);
   auto f32 = x.options().dtype(torch::kFloat32);
-  auto dgamma = torch::zeros({H}, f32), dbeta = torch::zeros({H}, f32);
-  if (rows == 0) return {dx, dgamma, dbeta};
+  if (rows == 0) return {dx, torch::zeros({H}, f32), torch::zeros({H}, f32)};
+  auto dgamma = torch::empty({H}, f32), dbeta = torch::empty({H}, f32);
   const int grid = bwd_grid(rows);
   auto scratch = torch::empty({2, grid, H}, f32);
   auto stream = at::cuda::getCurrentCUDAStream();
   float* pdg = scratch.data_ptr<float>();
   float* pdb = pdg + static_cast<size_t>(grid) * H;
-  ln_bwd_launch<0>(dy, x, mean.data_ptr<float>(), rstd.data_ptr<float>(), fptr(gamma), dx.data_ptr(), nullptr, pdg, pdb,
-                   grid, static_cast<float>(H), stream);
-  colsum2_kernel<<<(H + 255) / 256, 256, 0, stream>>>(pdg, pdb, dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), grid, H);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  ln_bwd_launch<0>(dy, x, mean.data_ptr<float>(), rstd.data_ptr<float>(), fptr(gamma),
+                   dres != nullptr ? dres->data_ptr() : nullptr, dx.data_ptr(), nullptr, pdg, pdb, grid,
+                   static_cast<float>(H), stream);
+  colsum_launch(pdg, pdb, dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), grid, H, stream);
   return {dx, dgamma, dbeta};
+}
+
+std::vector<torch::Tensor> layer_norm_bwd(torch::Tensor dy, torch::Tensor x, torch::Tensor mean, torch::Tensor rstd,
+                                          torch::Tensor gamma) {
+  return layer_norm_bwd_cta(dy, x, mean, rstd, gamma, nullptr);
 }
 
 std::vector<torch::Tensor> norm_bwd_partials(torch::Tensor dy, torch::Tensor x, torch::Tensor mean, torch::Tensor rstd,
@@ -553,17 +683,17 @@ std::vector<torch::Tensor> norm_bwd_partials(torch::Tensor dy, torch::Tensor x, 
   const int rows = x.size(0), H = x.size(1);
   auto f32 = x.options().dtype(torch::kFloat32);
   auto sums = torch::empty({rows, 2}, f32);
-  auto dgamma = torch::zeros({H}, f32), dbeta = torch::zeros({H}, f32);
-  if (rows == 0) return {sums, dgamma, dbeta};
+  if (rows == 0) return {sums, torch::zeros({H}, f32), torch::zeros({H}, f32)};
+  gamma = aligned16(gamma);
+  auto dgamma = torch::empty({H}, f32), dbeta = torch::empty({H}, f32);
   const int grid = bwd_grid(rows);
   auto scratch = torch::empty({2, grid, H}, f32);
   auto stream = at::cuda::getCurrentCUDAStream();
   float* pdg = scratch.data_ptr<float>();
   float* pdb = pdg + static_cast<size_t>(grid) * H;
-  ln_bwd_launch<1>(dy, x, mean.data_ptr<float>(), rstd.data_ptr<float>(), fptr(gamma), nullptr, sums.data_ptr<float>(), pdg,
+  ln_bwd_launch<1>(dy, x, mean.data_ptr<float>(), rstd.data_ptr<float>(), fptr(gamma), nullptr, nullptr, sums.data_ptr<float>(), pdg,
                    pdb, grid, 1.f, stream);
-  colsum2_kernel<<<(H + 255) / 256, 256, 0, stream>>>(pdg, pdb, dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), grid, H);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  colsum_launch(pdg, pdb, dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), grid, H, stream);
   return {sums, dgamma, dbeta};
 }
 
@@ -576,7 +706,8 @@ torch::Tensor norm_bwd_apply(torch::Tensor dy, torch::Tensor x, torch::Tensor me
   auto dx = torch::empty_like(x);
   if (rows == 0) return dx;
   auto stream = at::cuda::getCurrentCUDAStream();
-  ln_bwd_launch<2>(dy, x, mean.data_ptr<float>(), rstd.data_ptr<float>(), fptr(gamma), dx.data_ptr(), sums.data_ptr<float>(),
+  gamma = aligned16(gamma);
+  ln_bwd_launch<2>(dy, x, mean.data_ptr<float>(), rstd.data_ptr<float>(), fptr(gamma), nullptr, dx.data_ptr(), sums.data_ptr<float>(),
                    nullptr, nullptr, row_grid(rows), static_cast<float>(hidden), stream);
   return dx;
 }
@@ -609,24 +740,23 @@ std::vector<torch::Tensor> layer_norm_fwd_res(torch::Tensor x, c10::optional<tor
   check_rows(x);
   const bool has_res = residual.has_value() && residual->defined();
   const int rows = x.size(0), H = x.size(1);
-  TORCH_CHECK(gamma.scalar_type() == torch::kFloat32 && beta.scalar_type() == torch::kFloat32 && gamma.is_contiguous() &&
-              beta.is_contiguous() && gamma.numel() == H && beta.numel() == H, "norm parameters must be contiguous fp32 [H]");
+  TORCH_CHECK((gamma.scalar_type() == torch::kFloat32 || gamma.scalar_type() == x.scalar_type()) &&
+              beta.scalar_type() == gamma.scalar_type() && gamma.is_contiguous() && beta.is_contiguous() &&
+              gamma.numel() == H && beta.numel() == H, "norm parameters must be contiguous [H], fp32 or of the rows' type");
+  // A CTA per row for wide rows, and for so few that eight rows per CTA leave most SMs without one (decoding: 8 rows of 2048
+  // took 9.2 us on one SM, every vector of a row in the same 32 lanes; 2.4 us now).
+  const bool cta = !warp_path(x) || rows <= 2 * at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   torch::Tensor sum;
   if (has_res) {
     check_rows(*residual);
     TORCH_CHECK(residual->sizes() == x.sizes() && residual->scalar_type() == x.scalar_type());
-    if (!warp_path(x)) {                       // wide rows: separate add, then the CTA-per-row kernel
-      sum = x + *residual;
-      auto r = layer_norm_fwd(sum, gamma, beta, eps);
-      r.push_back(sum);
-      return r;
-    }
+    if (cta) return layer_norm_fwd_cta(x, &*residual, gamma, beta, eps);
     sum = torch::empty_like(x);
-  } else if (!warp_path(x)) {
-    auto r = layer_norm_fwd(x, gamma, beta, eps);
-    r.push_back(torch::Tensor());
-    return r;
+  } else if (cta) {
+    return layer_norm_fwd_cta(x, nullptr, gamma, beta, eps);
   }
+  gamma = aligned16(gamma);
+  beta = aligned16(beta);
   auto y = torch::empty_like(x);
   auto mean = torch::empty({rows}, x.options().dtype(torch::kFloat32));
   auto rstd = torch::empty({rows}, x.options().dtype(torch::kFloat32));
@@ -634,18 +764,18 @@ std::vector<torch::Tensor> layer_norm_fwd_res(torch::Tensor x, c10::optional<tor
   auto stream = at::cuda::getCurrentCUDAStream();
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   const int grid = std::max(1, std::min((rows + kWarpRows - 1) / kWarpRows, sms * 6));
-  if (has_res) {
-    DISPATCH_16_NV(x, ln_fwd_warp_kernel<T, NV, true><<<grid, 32 * kWarpRows, 0, stream>>>(
-                          reinterpret_cast<const T*>(x.data_ptr()), reinterpret_cast<const T*>(residual->data_ptr()),
-                          gamma.data_ptr<float>(), beta.data_ptr<float>(), reinterpret_cast<T*>(sum.data_ptr()),
-                          reinterpret_cast<T*>(y.data_ptr()), mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, H,
-                          static_cast<float>(eps));)
-  } else {
-    DISPATCH_16_NV(x, ln_fwd_warp_kernel<T, NV, false><<<grid, 32 * kWarpRows, 0, stream>>>(
-                          reinterpret_cast<const T*>(x.data_ptr()), nullptr, gamma.data_ptr<float>(), beta.data_ptr<float>(),
-                          nullptr, reinterpret_cast<T*>(y.data_ptr()), mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, H,
-                          static_cast<float>(eps));)
-  }
+#define LAUNCH_LN_FWD(RES, P)                                                                                             \
+  ln_fwd_warp_kernel<T, NV, RES, P><<<grid, 32 * kWarpRows, 0, stream>>>(                                                 \
+      reinterpret_cast<const T*>(x.data_ptr()), RES ? reinterpret_cast<const T*>(residual->data_ptr()) : nullptr,         \
+      reinterpret_cast<const P*>(gamma.data_ptr()), reinterpret_cast<const P*>(beta.data_ptr()),                          \
+      RES ? reinterpret_cast<T*>(sum.data_ptr()) : nullptr, reinterpret_cast<T*>(y.data_ptr()), mean.data_ptr<float>(),   \
+      rstd.data_ptr<float>(), rows, H, static_cast<float>(eps))
+  const bool f32 = gamma.scalar_type() == torch::kFloat32;
+  DISPATCH_16_NV(x, {
+    if (has_res) { if (f32) LAUNCH_LN_FWD(true, float); else LAUNCH_LN_FWD(true, T); }
+    else { if (f32) LAUNCH_LN_FWD(false, float); else LAUNCH_LN_FWD(false, T); }
+  })
+#undef LAUNCH_LN_FWD
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   return {y, mean, rstd, sum};
 }
@@ -656,21 +786,18 @@ std::vector<torch::Tensor> layer_norm_bwd_res(torch::Tensor dy, torch::Tensor x,
   check_rows(x);
   check_rows(dy);
   const bool has_res = dres.has_value() && dres->defined();
-  if (!warp_path(x)) {
-    auto r = layer_norm_bwd(dy, x, mean, rstd, gamma);
-    if (has_res) r[0].add_(*dres);
-    return r;
-  }
-  const int rows = x.size(0), H = x.size(1);
-  TORCH_CHECK(gamma.scalar_type() == torch::kFloat32 && gamma.is_contiguous() && gamma.numel() == H);
   if (has_res) {
     check_rows(*dres);
     TORCH_CHECK(dres->sizes() == x.sizes() && dres->scalar_type() == x.scalar_type());
   }
+  if (!warp_path(x)) return layer_norm_bwd_cta(dy, x, mean, rstd, gamma, has_res ? &*dres : nullptr);
+  const int rows = x.size(0), H = x.size(1);
+  TORCH_CHECK(gamma.scalar_type() == torch::kFloat32 && gamma.is_contiguous() && gamma.numel() == H);
+  gamma = aligned16(gamma);
   auto dx = torch::empty_like(x);
   auto f32 = x.options().dtype(torch::kFloat32);
-  auto dgamma = torch::zeros({H}, f32), dbeta = torch::zeros({H}, f32);
-  if (rows == 0) return {dx, dgamma, dbeta};
+  if (rows == 0) return {dx, torch::zeros({H}, f32), torch::zeros({H}, f32)};
+  auto dgamma = torch::empty({H}, f32), dbeta = torch::empty({H}, f32);
   auto stream = at::cuda::getCurrentCUDAStream();
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   const int grid = std::max(1, std::min((rows + kWarpRows - 1) / kWarpRows, 2 * sms));
@@ -688,8 +815,7 @@ std::vector<torch::Tensor> layer_norm_bwd_res(torch::Tensor dy, torch::Tensor x,
                                                         pdg, pdb, rows, H));)
   }
   C10_CUDA_KERNEL_LAUNCH_CHECK();
-  colsum2_kernel<<<(H + 255) / 256, 256, 0, stream>>>(pdg, pdb, dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), grid, H);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  colsum_launch(pdg, pdb, dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), grid, H, stream);
   return {dx, dgamma, dbeta};
 }
 

@@ -38,6 +38,31 @@ def test_act_backward_stripes(M, N, act):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,H", [(1, 2056), (300, 4096), (1200, 5120), (5, 6144), (7, 8200), (3, 16384)])
+def test_wide_layer_norm_with_residual(rows, H, dtype):
+    ops, _ = _ops()
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    x, r, dy, ds = (torch.randn(rows, H, generator=g, device="cuda").to(dtype) for _ in range(4))
+    flat = torch.randn(2 * H + 1, generator=g, device="cuda")
+    gamma, beta = flat[1:H + 1], flat[H + 1:]                      # views that start 4 bytes off a 16-byte boundary
+    y, mean, rstd, total = ops.layer_norm_fwd(x, gamma, beta, 1e-5, residual=r)
+    assert torch.equal(total, x + r)
+    t = total.double().requires_grad_(True)
+    gd, bd = gamma.double().requires_grad_(True), beta.double().requires_grad_(True)
+    ref = torch.nn.functional.layer_norm(t, (H, ), gd, bd, 1e-5)
+    ref.backward(dy.double())
+    assert ((y.double() - ref).abs() <= UNIT[dtype] * ref.abs() + 1e-5).all()
+    dx, dg, db = ops.layer_norm_bwd(dy, total, mean, rstd, gamma, dres=ds)
+    want = t.grad + ds.double()
+    assert ((dx.double() - want).abs() <= UNIT[dtype] * want.abs() + 1e-5).all()
+    # fp32 sums over the rows of terms below 36
+    bound = rows * 2.0**-24 * 36 * rows + 1e-4
+    assert ((dg.double() - gd.grad).abs() <= bound).all() and ((db.double() - bd.grad).abs() <= bound).all()
+    y2, _, _ = ops.layer_norm_fwd(total, gamma, beta, 1e-5)
+    assert torch.equal(y2, y)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("trans_a,trans_b", [(False, True), (False, False), (True, False), (True, True)])
 @pytest.mark.parametrize("M,N,K", [
     (256, 256, 64),            # one tile, one k-block
