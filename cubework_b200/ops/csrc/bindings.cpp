@@ -100,12 +100,16 @@ std::vector<torch::Tensor> gemm(torch::Tensor a, torch::Tensor b, bool trans_a, 
   if (M == 0 || N == 0) return {out, z};
   if (K == 0) { out.zero_(); return {out, z}; }
   torch::Tensor bias_f;
-  if (bias.has_value() && bias->defined()) {
+  GemmArgs g;
+  const bool skinny = !trans_a && trans_b && !out_f32 && M <= kSkinnyRows;      // the rule of gemm_launch
+  if (skinny && bias.has_value() && bias->defined() && bias->scalar_type() == a.scalar_type() && bias->is_contiguous()) {
+    TORCH_CHECK(bias->numel() == N && bias->is_cuda(), "bias must have one value per output column");
+    g.bias16 = bias->data_ptr();
+  } else if (bias.has_value() && bias->defined()) {
     bias_f = bias->to(torch::kFloat32).contiguous();
     TORCH_CHECK(bias_f.numel() == N, "bias must have one value per output column");
   }
   ensure_status();
-  GemmArgs g;
   g.a = a.data_ptr(); g.b = b.data_ptr(); g.out = out.data_ptr();
   g.z_out = want_z ? z.data_ptr() : nullptr;
   g.bias = bias_f.defined() ? bias_f.data_ptr<float>() : nullptr;

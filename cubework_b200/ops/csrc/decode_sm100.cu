@@ -9,7 +9,7 @@
 // merged by shuffles, warps through shared memory, CTAs through distributed shared memory, so the kernel needs neither
 // a workspace nor a counter that outlives the launch.
 // OPT-1.3B (24 layers of 32 heads x 64), 8 sequences of 1000 keys, one token: 15.3 ms -> 6.0 ms a pass together with the
-// GEMM below; concatenation alone ran at 1 TB/s (6.3 ms) and the fp32 copies of both caches took 2.2 ms.
+// GEMM below, of which the GPU works 2.0; concatenation alone ran at 1 TB/s (6.3 ms) and the fp32 copies of both caches took 2.2 ms.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -44,7 +44,7 @@ __device__ __forceinline__ float part_weight(float m, float l, float m_all) { re
 
 // LPK lanes share a key, 8 elements each.
 template <typename T, int LPK>
-__global__ void __launch_bounds__(kDecThreads) decode_attention_kernel(DecodeParams p) {
+__global__ void __launch_bounds__(kDecThreads, 2) decode_attention_kernel(DecodeParams p) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ float s_m[kDecWarps], s_l[kDecWarps];
@@ -246,14 +246,16 @@ std::vector<torch::Tensor> decode_attention(torch::Tensor qkv, torch::Tensor k_p
   p.bias = bias.defined() ? bias.data_ptr<float>() : nullptr;
   p.heads = static_cast<int>(H); p.T = static_cast<int>(T); p.dh = static_cast<int>(dh);
   p.scale = static_cast<float>(scale);
-  // CTAs per (sequence, head): enough for four per SM, but not more than there are rounds of keys to share
+  // CTAs per (sequence, head): as many as are resident at once (two per SM), but not more than there are rounds of keys to
+  // share.  A second wave costs more than it balances: start, query load, merge and two cluster barriers are about 8 us of
+  // a CTA's life (256 heads x 1001 keys of 64 with four CTAs each: 50 us, with one: 42; the traffic takes 20).
   const int lanes = static_cast<int>((dh + 7) / 8);
   const int lpk = lanes <= 4 ? 4 : (lanes <= 8 ? 8 : (lanes <= 16 ? 16 : 32));
   const int64_t round = static_cast<int64_t>(kDecWarps) * (32 / lpk) * kDecUnroll;
   const int64_t rounds = (T + 1 + round - 1) / round;
-  const int64_t want = 4 * at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  const int64_t room = 2 * at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   int ranks = 1;
-  while (ranks < 8 && ranks * B * H < want && ranks < rounds) ranks *= 2;
+  while (ranks < 8 && 2 * ranks * B * H <= room && ranks < rounds) ranks *= 2;
   auto stream = at::cuda::getCurrentCUDAStream();
   if (qkv.scalar_type() == torch::kBFloat16) dispatch_decode<__nv_bfloat16>(p, static_cast<int>(B * H), ranks, stream);
   else dispatch_decode<__half>(p, static_cast<int>(B * H), ranks, stream);
@@ -264,7 +266,7 @@ std::vector<torch::Tensor> decode_attention(torch::Tensor qkv, torch::Tensor k_p
 // y[M, N] = act(x[M, K] W[N, K]^T + b) for a handful of rows (M <= 32): one read of the weights is all the work there
 // is.  The persistent tcgen05 kernel has one tile per 256 weight rows (8 CTAs for N = 2048) and cannot ask for enough
 // bytes at a time.  Here a warp owns 16 weight rows as the M side of mma.m16n8k16 and the tokens are its N side; the
-// eight warps of a CTA split K between them in chunks of 64 elements and are added up in shared memory (a fixed order).
+// warps of a CTA split K between them in chunks of 64 elements and are added up in shared memory (a fixed order).
 // The k index of an MMA is summed over, so any bijection of it may be used as long as both operands share it: lane t
 // of a quad takes 8 consecutive elements (one 16-byte load) of a row, which are four k pairs of two MMAs.  Weights go
 // straight from global memory to registers; nothing is staged.
@@ -289,15 +291,15 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
   return v;
 }
 
-constexpr int kSkWarps = 8;
 constexpr int kSkChunk = 64;             // k elements of a warp's step: 128 bytes of every weight row
 
-template <typename T, int NT>            // NT groups of 8 tokens
-__global__ void __launch_bounds__(32 * kSkWarps) skinny_gemm_kernel(const T* __restrict__ x, const T* __restrict__ w,
-                                                                    const float* __restrict__ bias, T* __restrict__ y,
+template <typename T, int NT, int W>     // NT groups of 8 tokens, W warps
+__global__ void __launch_bounds__(32 * W) skinny_gemm_kernel(const T* __restrict__ x, const T* __restrict__ w,
+                                                                    const float* __restrict__ bias,
+                                                                    const T* __restrict__ bias16, T* __restrict__ y,
                                                                     T* __restrict__ z, int M, int N, int K, int act) {
   constexpr int U = NT == 1 ? 4 : (NT == 2 ? 2 : 1);        // steps in flight
-  __shared__ float red[kSkWarps][NT * 8][17];
+  __shared__ float red[W][NT * 8][17];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * 16;
@@ -309,13 +311,13 @@ __global__ void __launch_bounds__(32 * kSkWarps) skinny_gemm_kernel(const T* __r
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 
-  for (int k0 = warp * kSkChunk; k0 < K; k0 += kSkWarps * kSkChunk * U) {
+  for (int k0 = warp * kSkChunk; k0 < K; k0 += W * kSkChunk * U) {
     uint4 a[U][2][2], b[U][2][NT];
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const int k = k0 + u * kSkWarps * kSkChunk + s * 32 + t * 8;
+        const int k = k0 + u * W * kSkChunk + s * 32 + t * 8;
         const bool ok = k < K;                              // K is a multiple of 8
         a[u][s][0] = ok ? ldg_stream(w0 + k) : make_uint4(0, 0, 0, 0);
         a[u][s][1] = ok ? ldg_stream(w1 + k) : make_uint4(0, 0, 0, 0);
@@ -343,13 +345,14 @@ __global__ void __launch_bounds__(32 * kSkWarps) skinny_gemm_kernel(const T* __r
     red[warp][i * 8 + 2 * t + 1][g + 8] = acc[i][3];
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < NT * 8 * 16; e += 32 * kSkWarps) {
+  for (int e = threadIdx.x; e < NT * 8 * 16; e += 32 * W) {
     const int m = e >> 4, c = e & 15, n = n0 + c;
     if (m >= M || n >= N) continue;
     float v = 0.f;
 #pragma unroll
-    for (int q = 0; q < kSkWarps; ++q) v += red[q][m][c];
+    for (int q = 0; q < W; ++q) v += red[q][m][c];
     if (bias != nullptr) v += __ldg(bias + n);
+    else if (bias16 != nullptr) v += to_f(bias16[n]);
     const size_t at = static_cast<size_t>(m) * N + n;
     if (z != nullptr) z[at] = from_f<T>(v);
     if (act == kActGelu) v = gelu_fast(v);
@@ -363,11 +366,16 @@ static void launch_skinny(const GemmArgs& g, cudaStream_t stream) {
   const int grid = (g.N + 15) / 16;
   const T* x = reinterpret_cast<const T*>(g.a);
   const T* w = reinterpret_cast<const T*>(g.b);
+  const T* b16 = reinterpret_cast<const T*>(g.bias16);
   T* y = reinterpret_cast<T*>(g.out);
   T* z = reinterpret_cast<T*>(g.z_out);
-  if (g.M <= 8) skinny_gemm_kernel<T, 1><<<grid, 32 * kSkWarps, 0, stream>>>(x, w, g.bias, y, z, g.M, g.N, g.K, g.act);
-  else if (g.M <= 16) skinny_gemm_kernel<T, 2><<<grid, 32 * kSkWarps, 0, stream>>>(x, w, g.bias, y, z, g.M, g.N, g.K, g.act);
-  else skinny_gemm_kernel<T, 4><<<grid, 32 * kSkWarps, 0, stream>>>(x, w, g.bias, y, z, g.M, g.N, g.K, g.act);
+  // 16 warps share a long K: with eight, each made four dependent rounds of loads at K = 8192 (2048 x 8192 weights: 9.7 us)
+#define LAUNCH_SKINNY(NT, W) \
+  skinny_gemm_kernel<T, NT, W><<<grid, 32 * W, 0, stream>>>(x, w, g.bias, b16, y, z, g.M, g.N, g.K, g.act)
+  if (g.M <= 8) { if (g.K >= 4096) LAUNCH_SKINNY(1, 16); else LAUNCH_SKINNY(1, 8); }
+  else if (g.M <= 16) { if (g.K >= 4096) LAUNCH_SKINNY(2, 16); else LAUNCH_SKINNY(2, 8); }
+  else { if (g.K >= 4096) LAUNCH_SKINNY(4, 16); else LAUNCH_SKINNY(4, 8); }
+#undef LAUNCH_SKINNY
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 

@@ -13,6 +13,7 @@ struct GemmArgs {
   void* out;
   void* z_out = nullptr;
   const float* bias = nullptr;
+  const void* bias16 = nullptr;     // bias in the operands' type instead (skinny products only)
   int M, N, K;
   bool trans_a, trans_b;
   bool is_bf16 = true;
