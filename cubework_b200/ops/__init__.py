@@ -61,6 +61,8 @@ def shadow(param: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
         return param.detach()
     key = (id(param), dtype)
     s = _SHADOWS.get(key)
+    if s is not None and s.version == param._version and s.tensor.shape == param.shape and s.tensor.device == param.device:
+        return s.tensor
     base = param.detach()
     if s is None or s.tensor.shape != base.shape or s.tensor.device != base.device:
         s = _Shadow()
@@ -91,6 +93,39 @@ def _register_shadow_finalizer(param, key):
         weakref.finalize(param, _SHADOWS.pop, key, None)
     except TypeError:
         pass
+
+
+# ---------------------------------------------------------------------------------------------------
+# layers whose autograd node is native (ops/csrc/native_layers.cpp)
+# ---------------------------------------------------------------------------------------------------
+_ACT_CODE = {None: 0, "gelu": 1, "relu": 2}
+
+
+def _native(x, cd) -> bool:
+    """The native nodes take CUDA tensors with a 16-bit compute dtype, outside function transforms (which refuse the Python
+    functions and would not see the native ones)."""
+    if not (x.is_cuda and cd in _LOWP and kernels_enabled()) or torch._C._are_functorch_transforms_active():
+        return False
+    ext.require()
+    return True
+
+
+def native_linear(x, w, b, w_is_out_in, act):
+    """``act(x @ op(w) + b)`` through the native node, or None when the Python function has to take it: extents that need
+    padding, a weight of another dtype, parameters whose storage is swapped between the passes."""
+    cd = compute_dtype(x)
+    if not _native(x, cd) or not w.is_cuda or w.dim() != 2 or (w.dtype != torch.float32 and w.dtype != cd) or \
+            (w.shape[0] | w.shape[1]) % 8 or act not in _ACT_CODE or getattr(w, "storage_is_swapped", False):
+        return None
+    return ext.require().native_linear(x, w, b, shadow(w, cd), w_is_out_in, _ACT_CODE[act])
+
+
+def native_norm(x, residual, gamma, beta, eps):
+    """``[LN(x)]`` or ``[x + residual, LN(x + residual)]`` through the native node, or None."""
+    cd = compute_dtype(x)
+    if not _native(x, cd) or not gamma.is_cuda or x.shape[-1] % 8 or x.shape[-1] > 16384:
+        return None
+    return ext.require().native_norm(x, residual, gamma, beta, eps, cd)
 
 
 # ---------------------------------------------------------------------------------------------------
@@ -315,6 +350,8 @@ def attention_packed(qkv: torch.Tensor, causal: bool, key_bias: Optional[torch.T
     B, T, H, D3 = qkv.shape
     dh = D3 // 3
     scale = scale if scale is not None else 1.0 / math.sqrt(dh)
+    if ext.ATTN_TRACE is None and _native(qkv, qkv.dtype):
+        return ext.require().native_attention(qkv.contiguous(), causal, key_bias, scale).view(B, T, H * dh)
     if use_kernels(qkv):
         return _AttentionFn.apply(qkv.contiguous(), causal, key_bias, scale).view(B, T, H * dh)
     q, k, v = qkv.permute(0, 2, 1, 3).chunk(3, dim=-1)

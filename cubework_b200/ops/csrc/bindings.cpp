@@ -50,6 +50,13 @@ bool attention_ready();
 // decode_sm100.cu
 std::vector<torch::Tensor> decode_attention(torch::Tensor qkv, torch::Tensor k_past, torch::Tensor v_past,
                                             c10::optional<torch::Tensor> key_bias, double scale);
+// native_layers.cpp
+torch::Tensor native_linear(const torch::Tensor& x, const torch::Tensor& w, const c10::optional<torch::Tensor>& b,
+                            const torch::Tensor& wc, bool out_in, int64_t act);
+std::vector<torch::Tensor> native_norm(const torch::Tensor& x, const c10::optional<torch::Tensor>& residual,
+                                       const torch::Tensor& gamma, const torch::Tensor& beta, double eps, torch::ScalarType cd);
+torch::Tensor native_attention(const torch::Tensor& qkv, bool causal, const c10::optional<torch::Tensor>& bias, double scale);
+int64_t native_launch_count();
 // comm.cu
 void register_comm(pybind11::module& m);
 
@@ -151,6 +158,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attention_fwd", &cw::attention_fwd);
   m.def("attention_bwd", &cw::attention_bwd);
   m.def("decode_attention", &cw::decode_attention);
+  m.def("native_linear", &cw::native_linear);
+  m.def("native_norm", &cw::native_norm);
+  m.def("native_attention", &cw::native_attention);
+  m.def("native_launch_count", &cw::native_launch_count);
   m.def("attention_ready", &cw::attention_ready);
   cw::register_comm(m);
 }

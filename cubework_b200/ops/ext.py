@@ -16,7 +16,7 @@ _launches = 0   # kernels of this package launched so far (bench.py reports the 
 
 
 def launch_count():
-    return _launches
+    return _launches + (_mod.native_launch_count() if _mod is not None else 0)
 
 
 def _count(n=1):

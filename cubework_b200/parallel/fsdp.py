@@ -59,6 +59,7 @@ class _FlatGroup:
         self.empty = torch.empty(0, dtype=flat.dtype, device=flat.device)
         for p in params:
             p.data = self.empty
+            p.storage_is_swapped = True     # nothing derived from it may be kept from the forward to the backward pass
 
     def gather(self):
         if self.full is not None:

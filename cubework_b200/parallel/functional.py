@@ -66,12 +66,14 @@ class _AddLayerNorm(torch.autograd.Function):
 
 
 def layer_norm(x, gamma, beta, eps):
-    return _LayerNorm.apply(x, gamma, beta, eps)
+    out = ops.native_norm(x, None, gamma, beta, eps)
+    return out[0] if out is not None else _LayerNorm.apply(x, gamma, beta, eps)
 
 
 def add_layer_norm(x, r, gamma, beta, eps):
     """``(x + r, LN(x + r))``."""
-    return _AddLayerNorm.apply(x, r, gamma, beta, eps)
+    out = ops.native_norm(x, r, gamma, beta, eps)
+    return tuple(out) if out is not None else _AddLayerNorm.apply(x, r, gamma, beta, eps)
 
 
 class _MaskedEmbedding(torch.autograd.Function):
@@ -140,4 +142,5 @@ class _LocalLinear(torch.autograd.Function):
 
 
 def local_linear(x, w, b=None, w_is_out_in=True, act=None):
-    return _LocalLinear.apply(x, w, b, w_is_out_in, act, torch.is_grad_enabled())
+    y = ops.native_linear(x, w, b, w_is_out_in, act)
+    return y if y is not None else _LocalLinear.apply(x, w, b, w_is_out_in, act, torch.is_grad_enabled())
