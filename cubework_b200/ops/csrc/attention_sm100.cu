@@ -3,12 +3,10 @@
 // this package and of the reference use: benchmark/gpt2/gpt2.py:66-96, vit/vit.py:74-89, opt/opt.py:70-128).
 // Scores never reach HBM; the reference materialises [b, heads, T, T] several times per layer.
 //
-// Forward, one CTA per (128-query block, head, batch), 128 threads, thread r owns query row r:
+// Forward, persistent CTAs that run two 128-query tiles at a time, thread r of a softmax group owns query row r:
 //   S = Q K^T         tcgen05.mma, both operands K-major in shared memory, accumulator in TMEM (128 columns)
-//   softmax           rows read back with tcgen05.ld, online max / sum in the exp2 domain, P written to shared
-//                     memory as 16-bit in the MMA's swizzled layout
-//   O_blk = P V       tcgen05.mma, V consumed as an MN-major operand straight from its row-major image
-//   O = O*alpha+O_blk in registers
+//   softmax           rows read back with tcgen05.ld, online max / sum in the exp2 domain, P as 16-bit back to TMEM
+//   O += P V          tcgen05.mma, V consumed as an MN-major operand straight from its row-major image; O stays in TMEM
 // Backward, one work item per (128-key block, head, batch) looping over query blocks: S and dP = dO V^T in TMEM,
 // P / dS written to shared memory, dV += P^T dO and dK += dS^T Q accumulate in TMEM across the loop,
 // dQ = dS K is added to an fp32 scratch buffer (several key blocks contribute to one query block).  Head dims up
@@ -28,7 +26,6 @@
 
 namespace cw {
 
-constexpr int kAttnThreads = 128;
 constexpr int kBlk = 128;                 // queries per CTA == keys per step
 constexpr float kLog2e = 1.4426950408889634f;
 // Descriptor offsets of an operand read "MN-major" from a row-major [rows, 64*NB] swizzled image.
@@ -111,234 +108,6 @@ __device__ __forceinline__ void tma_tile(uint8_t* img, const CUtensorMap* map, u
   for (int cb = 0; cb < NB; ++cb) tma_load_4d(img + cb * (kBlk * 128), map, bar, cb * 64, row0, h, b);
 }
 
-template <typename T, int DP>
-__global__ void __launch_bounds__(kAttnThreads)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                const __grid_constant__ CUtensorMap map_v, AttnParams p) {
-  constexpr int NB = (DP + 63) / 64;
-  constexpr int kImg = NB * kBlk * 128;          // bytes of a [128 x DP] image
-  constexpr uint32_t kTmemCols = 256;             // S: [0,128)  O_blk: [128, 128+DP)
-  constexpr bool kOnePass = DP <= 64;             // scores of the whole block fit in registers
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* q_img = smem;
-  uint8_t* k_img = q_img + kImg;
-  uint8_t* v_img = k_img + kImg;
-  uint8_t* p_img = v_img + kImg;                  // [128 x 128] 16-bit = 32 KB
-  uint64_t* bars = reinterpret_cast<uint64_t*>(p_img + 2 * kBlk * 128);   // 0:S 1:O 2:Q 3:K 4:V
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* s_bias = reinterpret_cast<float*>(tmem_slot + 2);                 // [2][128] key bias (log2 domain) of a block
-
-  const int r = threadIdx.x, warp = r >> 5;
-  const int qb = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-  const int q0 = qb * kBlk;
-  const float* kbias = p.key_bias != nullptr ? p.key_bias + static_cast<int64_t>(b) * p.T : nullptr;
-  if (kbias != nullptr) s_bias[r] = r < p.T ? kbias[r] * kLog2e : 0.f;
-
-  if (r == 0) {
-    for (int i = 0; i < 5; ++i) mbar_init(&bars[i], 1);
-    *abort_flag = 0;
-    fence_barrier_init();
-    mbar_expect_tx(&bars[2], kImg);
-    tma_tile<NB>(q_img, &map_q, &bars[2], q0, h, b);
-    mbar_expect_tx(&bars[3], kImg);
-    tma_tile<NB>(k_img, &map_k, &bars[3], 0, h, b);
-    mbar_expect_tx(&bars[4], kImg);
-    tma_tile<NB>(v_img, &map_v, &bars[4], 0, h, b);
-  }
-  if (warp == 0) {
-    __syncwarp();   // lane 0 just left the set-up branch: the allocation is warp-collective
-    tmem_alloc(tmem_slot, kTmemCols);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-  const uint32_t idesc_s = make_idesc_f16(kBlk, kBlk, false, false, p.is_bf16);
-  const uint32_t idesc_o = make_idesc_f16(kBlk, DP, false, true, p.is_bf16);
-
-  const int q_idx = q0 + r;
-  const float sc2 = p.scale * kLog2e;
-  float m_run = -INFINITY, l_run = 0.f;
-  float o_acc[DP];
-#pragma unroll
-  for (int i = 0; i < DP; ++i) o_acc[i] = 0.f;
-
-  const int n_kv = p.causal ? min((p.T + kBlk - 1) / kBlk, qb + 1) : (p.T + kBlk - 1) / kBlk;
-  bool ok = true;
-  for (int j = 0; j < n_kv && ok; ++j) {
-    const int k0 = j * kBlk;
-    if (r == 0) {
-      bool good = true;
-      if (j == 0) good = mbar_wait(&bars[2], 0, abort_flag, p.status, kErrAttnBarrierTimeout, blockIdx.x);
-      good = good && mbar_wait(&bars[3], j & 1, abort_flag, p.status, kErrAttnBarrierTimeout, blockIdx.x);
-      if (good) {
-        tc_fence_after();
-#pragma unroll
-        for (int k16 = 0; k16 < DP / 16; ++k16)
-          tc_mma_f16(tmem, kmajor_desc(smem_u32(q_img), k16), kmajor_desc(smem_u32(k_img), k16), idesc_s, k16 > 0);
-        tc_commit(&bars[0]);
-      }
-    }
-    if (!mbar_wait(&bars[0], j & 1, abort_flag, p.status, kErrAttnBarrierTimeout, blockIdx.x)) { ok = false; break; }
-    tc_fence_after();
-    if (r == 0 && j + 1 < n_kv) {                 // K is free again: fetch the next block behind the softmax
-      mbar_expect_tx(&bars[3], kImg);
-      tma_tile<NB>(k_img, &map_k, &bars[3], k0 + kBlk, h, b);
-    }
-    const bool diag = (p.causal && j == qb) || (k0 + kBlk > p.T);   // block needs element-wise masking
-    const float* bias_j = s_bias + (j & 1) * kBlk;
-    if (kbias != nullptr && j + 1 < n_kv) {       // bias of the next block; published by this iteration's __syncthreads
-      const int key = k0 + kBlk + r;
-      s_bias[((j + 1) & 1) * kBlk + r] = key < p.T ? kbias[key] * kLog2e : 0.f;
-    }
-    float alpha, l_blk = 0.f, m_use;
-    if (kOnePass) {
-      float sv[kBlk];
-      float m_blk = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t raw[32];
-        tmem_ld_32x32(tmem + lane_base + c * 32, raw);
-        tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int key = k0 + c * 32 + i;
-          float sx = __uint_as_float(raw[i]) * sc2;
-          if (kbias != nullptr) sx += bias_j[c * 32 + i];
-          if (diag && (key >= p.T || (p.causal && key > q_idx))) sx = -INFINITY;
-          sv[c * 32 + i] = sx;
-          m_blk = fmaxf(m_blk, sx);
-        }
-      }
-      const float m_new = fmaxf(m_run, m_blk);
-      m_use = (m_new == -INFINITY) ? 0.f : m_new;
-      alpha = (m_run == -INFINITY) ? 0.f : exp2f(m_run - m_use);
-      m_run = m_new;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float pv[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float e = exp2f(sv[c * 32 + i] - m_use);
-          pv[i] = e;
-          l_blk += e;
-        }
-        store_p_chunk<T>(p_img, r, c * 32, pv);
-      }
-    } else {
-      float m_blk = -INFINITY;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t raw[32];
-        tmem_ld_32x32(tmem + lane_base + c * 32, raw);
-        tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int key = k0 + c * 32 + i;
-          float sx = __uint_as_float(raw[i]) * sc2;
-          if (kbias != nullptr) sx += bias_j[c * 32 + i];
-          if (diag && (key >= p.T || (p.causal && key > q_idx))) sx = -INFINITY;
-          m_blk = fmaxf(m_blk, sx);
-        }
-      }
-      const float m_new = fmaxf(m_run, m_blk);
-      m_use = (m_new == -INFINITY) ? 0.f : m_new;
-      alpha = (m_run == -INFINITY) ? 0.f : exp2f(m_run - m_use);
-      m_run = m_new;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t raw[32];
-        tmem_ld_32x32(tmem + lane_base + c * 32, raw);
-        tmem_wait_ld();
-        float pv[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int key = k0 + c * 32 + i;
-          float sx = __uint_as_float(raw[i]) * sc2;
-          if (kbias != nullptr) sx += bias_j[c * 32 + i];
-          if (diag && (key >= p.T || (p.causal && key > q_idx))) sx = -INFINITY;
-          const float e = exp2f(sx - m_use);
-          pv[i] = e;
-          l_blk += e;
-        }
-        store_p_chunk<T>(p_img, r, c * 32, pv);
-      }
-    }
-    l_run = l_run * alpha + l_blk;
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    if (r == 0) {
-      if (mbar_wait(&bars[4], j & 1, abort_flag, p.status, kErrAttnBarrierTimeout, blockIdx.x)) {
-        tc_fence_after();
-#pragma unroll
-        for (int k16 = 0; k16 < kBlk / 16; ++k16)
-          tc_mma_f16(tmem + 128, kmajor_desc(smem_u32(p_img), k16), mnmajor_desc(smem_u32(v_img), k16), idesc_o, k16 > 0);
-        tc_commit(&bars[1]);
-      }
-    }
-    if (!mbar_wait(&bars[1], j & 1, abort_flag, p.status, kErrAttnBarrierTimeout, blockIdx.x)) { ok = false; break; }
-    tc_fence_after();
-    if (r == 0 && j + 1 < n_kv) {                 // V is free again
-      mbar_expect_tx(&bars[4], kImg);
-      tma_tile<NB>(v_img, &map_v, &bars[4], k0 + kBlk, h, b);
-    }
-#pragma unroll
-    for (int c = 0; c < DP / 32; ++c) {
-      uint32_t raw[32];
-      tmem_ld_32x32(tmem + 128 + lane_base + c * 32, raw);
-      tmem_wait_ld();
-#pragma unroll
-      for (int i = 0; i < 32; ++i) o_acc[c * 32 + i] = o_acc[c * 32 + i] * alpha + __uint_as_float(raw[i]);
-    }
-    tc_fence_before();
-  }
-
-  if (ok && q_idx < p.T) {
-    const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-    T* o = reinterpret_cast<T*>(p.out) + ((static_cast<int64_t>(b) * p.T + q_idx) * p.H + h) * p.dh;
-#pragma unroll
-    for (int d = 0; d < DP; ++d)
-      if (d < p.dh) o[d] = from_f<T>(o_acc[d] * inv);
-    p.lse[(static_cast<int64_t>(b) * p.H + h) * p.T + q_idx] = (l_run > 0.f) ? m_run + log2f(l_run) : -INFINITY;
-  }
-  if (*abort_flag) {
-    for (int i = 0; i < 32; ++i) __nanosleep(1000);
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) {
-    tc_fence_after();
-    tmem_dealloc(tmem, kTmemCols);
-  }
-}
-
-// ---------------------------------------------------------------------------------------------------------
-// Warp-specialised forward for head dims up to 64: persistent CTAs (one per SM) of ten warps.
-//   warps 0-3 / 4-7  two softmax groups; group w owns the key blocks j = w, w+2, ... of the current query tile,
-//                    with its own running max / sum and its own output accumulator, merged at the end of the tile
-//   warp 8           issues every tcgen05.mma: S_w = Q K_j^T into group w's score columns, O_w += P_w V_j
-//   warp 9           TMA producer: Q (two buffers), K and V (rings of three), key bias (ring of six)
-// While one group runs its exponentials the tensor core works for the other, and the next score block of a group
-// is issued as soon as its P has been handed over, so no group waits for a tensor-core round trip with nothing
-// else resident on the SM.  O accumulates in TMEM across key blocks; the owning group rescales it in place
-// (tcgen05.ld / st) before handing over the next P.  All hand-overs are mbarriers with bounded waits.
-// TMEM: S_0 [0,128)  S_1 [128,256)  O_0 [256,256+DP)  O_1 [320,320+DP).
-// ---------------------------------------------------------------------------------------------------------
-// Warp-specialised forward for head dims up to 64: persistent CTAs (one per SM) of twelve warps that run TWO
-// independent query tiles at a time ("lanes" w = 0, 1), each with its own
-//   softmax group   warps 4w .. 4w+3: thread r owns query row r; two passes over the scores in TMEM (maximum, then
-//                   exponentials), P to shared memory, O rescaled in TMEM, the tile's output written at the end
-//   MMA issuer      warp 8 + w:  S = Q K_j^T, then after the group hands over P_j: O += P_j V_j and S for block j+1
-//   TMA producer    warp 10 + w: Q, K (ring of two), V, key bias (ring of four)
-// While one lane waits for a tensor-core round trip or writes its output, the other lane's group computes, and the
-// MMA / TMA threads never sit on a softmax warp's critical path.  O accumulates in TMEM across key blocks; the group
-// rescales it in place (tcgen05.ld / st) before handing over the next P.  All hand-overs are mbarriers with bounded
-// waits.  TMEM: S_w at 128 w, O_w at 256 + 64 w.
 template <bool MASKED, bool BIAS>
 __device__ __forceinline__ float chunk_max(const uint32_t (&raw)[32], const float* bias, float sc2, int key0, int q_idx, int T,
                                            bool causal, float m) {
@@ -397,44 +166,66 @@ __device__ __forceinline__ bool mbar_wait_ol(uint64_t* bar, uint32_t parity, vol
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, abort_flag, status, detail);
 }
-constexpr int kWsThreads = 384;
-constexpr int kWsKRing = 2, kWsBiasRing = 4;
+// ---------------------------------------------------------------------------------------------------------
+// Forward: persistent CTAs of eleven warps that take two neighbouring query tiles ("lanes" w = 0, 1) of one (batch, head)
+// and share their K / V blocks.
+//   softmax group   warps 4w .. 4w+3: thread r owns query row r; two passes over the scores in TMEM (maximum, then
+//                   exponentials); P goes back to TMEM as 16 bits and is the A operand of P V from there
+//   MMA issuers     warps 8, 9: S_w = Q_w K_j^T and O_w += P_w V_j
+//   TMA producer    warp 10: Q_w, one ring of four stages that K and V blocks share, key bias (ring of four)
+// What bounds it: 128 x 128 scores take 1024 clocks of the exponential units, and at a head dim of 128 the two products as
+// many of the tensor cores.  Two lanes keep both busy: while one group waits for a product the other computes.
+//   head dim <= 64  P has TMEM columns of its own, so the next scores are computed while the group still works on the last
+//   head dim > 64   S and O of two lanes fill TMEM; P lies over the first half of the scores it came from, and the next
+//                   scores follow once P V has finished with it
+// OPT-13B layer (4 x 40 heads x 2048 x 128, causal): 2121 us with one tile per CTA and a thread per row that did everything in
+// sequence, 0.28 to 0.43 ms now; ViT-B 256 x 12 heads x 197 x 64: 304 -> 204 us (four-warp groups with P through shared memory,
+// K and V fetched per tile); 32 x 64 heads x 1024 x 25: 1124 -> 1048.
+// P through shared memory would need 32 KB per lane (no room at 128) and a second operand at the shared memory's rate.
+// O accumulates in TMEM and is rescaled only when the running maximum has grown by more than 2^8 (kRescaleLog2): until
+// then P is relative to the older maximum, which is exact up to the same relative rounding, and stays below 256.
+// TMEM: S_w at 128 w; head dim <= 64: O_w at 256 + 64 w, P_w at 384 + 64 w; above: P_w at 128 w, O_w at 256 + 128 w.
+constexpr int kFwdThreads = 352;
+constexpr int kFwdRing = 4, kFwdBiasRing = 4;
+constexpr float kRescaleLog2 = 8.f;
 template <int DP>
-constexpr int fwd_ws_smem() {
-  return 2 * ((1 + kWsKRing + 1) * kBlk * 128 + 2 * kBlk * 128 + kWsBiasRing * kBlk * 4) + 768 + 1024;
+constexpr int fwd_stage_bytes() { return DP <= 64 ? 8 * 32 * DP * 2 : 0; }     // output rows that are no multiple of 16 bytes
+template <int DP>
+constexpr int fwd_smem() {
+  return (2 + kFwdRing) * ((DP + 63) / 64) * kBlk * 128 + fwd_stage_bytes<DP>() + kFwdBiasRing * kBlk * 4 + 512 + 1024;
 }
-
-struct WsLaneBars {
-  uint64_t q_full, q_empty;
-  uint64_t k_full[kWsKRing], k_empty[kWsKRing];
-  uint64_t v_full, v_empty;
-  uint64_t s_full, s_free, p_ready, o_full;
-  int bias_nz[kWsBiasRing];        // the key bias of this ring slot has a non-zero entry
+struct FwdBars {
+  uint64_t q_full[2], q_empty[2];
+  uint64_t kv_full[kFwdRing], kv_empty[kFwdRing];
+  uint64_t s_full[2], s_free[2], p_ready[2], o_full[2];
+  int bias_nz[kFwdBiasRing];       // the key bias of this ring slot has a non-zero entry
 };
 
 template <typename T, int DP>
-__global__ void __launch_bounds__(kWsThreads, 1)
-attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                   const __grid_constant__ CUtensorMap map_v, AttnParams p) {
-  static_assert(DP <= 64, "one 64-column image per operand");
-  constexpr int kImg = kBlk * 128;                 // 16 KB: a [128 x 64] 16-bit image
-  constexpr int kPImg = 2 * kBlk * 128;            // 32 KB: a [128 x 128] 16-bit image
-  constexpr int kLaneBytes = (1 + kWsKRing + 1) * kImg + kPImg + kWsBiasRing * kBlk * 4;
+__global__ void __launch_bounds__(kFwdThreads, 1)
+attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                const __grid_constant__ CUtensorMap map_v, AttnParams p) {
+  constexpr int NB = (DP + 63) / 64;
+  constexpr int kImg = NB * kBlk * 128;            // a [128 x 64 NB] 16-bit image
+  constexpr bool kOwnP = DP <= 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  WsLaneBars* all_bars = reinterpret_cast<WsLaneBars*>(smem + 2 * kLaneBytes);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(all_bars + 2);
+  uint8_t* q_img = smem;                           // [2]
+  uint8_t* kv_img = smem + 2 * kImg;               // [kFwdRing]
+  uint8_t* out_stage = kv_img + kFwdRing * kImg;
+  float* s_bias = reinterpret_cast<float*>(out_stage + fwd_stage_bytes<DP>());     // [kFwdBiasRing][128], log2 domain
+  FwdBars* bars = reinterpret_cast<FwdBars*>(s_bias + kFwdBiasRing * kBlk);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int w = 0; w < 2; ++w) {
-      WsLaneBars* bb = all_bars + w;
-      mbar_init(&bb->q_full, 1); mbar_init(&bb->q_empty, 1);
-      for (int i = 0; i < kWsKRing; ++i) { mbar_init(&bb->k_full[i], 1); mbar_init(&bb->k_empty[i], 1); }
-      mbar_init(&bb->v_full, 1); mbar_init(&bb->v_empty, 1);
-      mbar_init(&bb->s_full, 1); mbar_init(&bb->s_free, kBlk); mbar_init(&bb->p_ready, kBlk); mbar_init(&bb->o_full, 1);
+      mbar_init(&bars->q_full[w], 1); mbar_init(&bars->q_empty[w], 1);
+      mbar_init(&bars->s_full[w], 1); mbar_init(&bars->s_free[w], kBlk);
+      mbar_init(&bars->p_ready[w], kBlk); mbar_init(&bars->o_full[w], 1);
     }
+    for (int i = 0; i < kFwdRing; ++i) { mbar_init(&bars->kv_full[i], 1); mbar_init(&bars->kv_empty[i], kOwnP ? 2 : 1); }   // issuers
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -448,157 +239,198 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  // this thread's lane and that lane's buffers
-  const int w = warp < 8 ? warp >> 2 : (warp - 8) & 1;
-  uint8_t* lane_smem = smem + w * kLaneBytes;
-  uint8_t* q_img = lane_smem;
-  uint8_t* k_img = q_img + kImg;                   // [kWsKRing]
-  uint8_t* v_img = k_img + kWsKRing * kImg;
-  uint8_t* p_img = v_img + kImg;
-  float* s_bias = reinterpret_cast<float*>(p_img + kPImg);          // [kWsBiasRing][128], log2 domain
-  WsLaneBars* bars = all_bars + w;
-  const uint32_t tm_s = tmem + w * 128, tm_o = tmem + 256 + w * 64;
-
   const int n_qb = (p.T + kBlk - 1) / kBlk;
+  const int n_pair = (n_qb + 1) / 2;
   const int bh_total = p.B * p.H;
-  const int tiles = n_qb * bh_total;
-  auto n_kv_of = [&](int qb) { return p.causal ? min(n_qb, qb + 1) : n_qb; };
-  // tiles of this lane, heaviest (most key blocks) first: t = first, first + stride, ...
-  const int first = blockIdx.x + w * gridDim.x, stride = 2 * gridDim.x;
+  const int items = n_pair * bh_total;
+  // key blocks of a tile; 0 when the pair has no such tile.  Lane 0 never has more than lane 1 unless lane 1 has none.
+  auto n_kv_of = [&](int qb) { return qb >= n_qb ? 0 : (p.causal ? qb + 1 : n_qb); };
+  const int first = blockIdx.x, stride = gridDim.x;         // heaviest pairs first
 
-  if (warp >= 10) {
+  if (warp == 10) {
     // =========================================================================== TMA producer (+ key bias)
-    int kcount = 0, vcount = 0, tile_it = 0;
-    for (int t = first; t < tiles; t += stride, ++tile_it) {
+    int kv = 0, kcount = 0;
+    int q_use[2] = {0, 0};
+    for (int t = first; t < items; t += stride) {
       if (__shfl_sync(0xffffffffu, lane == 0 ? *abort_flag : 0, 0)) break;     // one decision for the whole warp
-      const int qb = n_qb - 1 - t / bh_total, bh = t % bh_total;
+      const int qb0 = 2 * (n_pair - 1 - t / bh_total), bh = t % bh_total;
       const int h = bh % p.H, b = bh / p.H;
-      const int n_kv = n_kv_of(qb);
+      const int n_kv = max(n_kv_of(qb0), n_kv_of(qb0 + 1));
       bool ok = true;
-      if (lane == 0) {
-        ok = mbar_wait_ol(&bars->q_empty, (tile_it & 1) ^ 1, abort_flag, p.status, t);
-        if (ok) {
-          mbar_expect_tx(&bars->q_full, kImg);
-          tma_load_4d(q_img, &map_q, &bars->q_full, 0, qb * kBlk, h, b);
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        if (qb0 + w >= n_qb) continue;
+        if (lane == 0 && ok) {
+          ok = mbar_wait_ol(&bars->q_empty[w], (q_use[w] & 1) ^ 1, abort_flag, p.status, t);
+          if (ok) {
+            mbar_expect_tx(&bars->q_full[w], kImg);
+            tma_tile<NB>(q_img + w * kImg, &map_q, &bars->q_full[w], (qb0 + w) * kBlk, h, b);
+          }
         }
+        ++q_use[w];
       }
       for (int j = 0; j < n_kv; ++j) {
-        const int ks = kcount % kWsKRing;
-        if (lane == 0)
-          ok = ok && mbar_wait_ol(&bars->k_empty[ks], ((kcount / kWsKRing) & 1) ^ 1, abort_flag, p.status, t);
+        const int ks = kv % kFwdRing, kp = (kv / kFwdRing) & 1;
+        if (lane == 0) ok = ok && mbar_wait_ol(&bars->kv_empty[ks], kp ^ 1, abort_flag, p.status, t);
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
         if (p.key_bias != nullptr) {
-          float* dst = s_bias + (kcount % kWsBiasRing) * kBlk;
+          // slot j % 4 was last read for block j - 4; both groups were done with block j - 3 before this stage became free
+          float* dst = s_bias + (kcount % kFwdBiasRing) * kBlk;
+          bool nz = false;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int key = j * kBlk + lane * 4 + i;
-            dst[lane * 4 + i] = key < p.T ? p.key_bias[static_cast<int64_t>(b) * p.T + key] * kLog2e : 0.f;
+            const float v = key < p.T ? p.key_bias[static_cast<int64_t>(b) * p.T + key] * kLog2e : 0.f;
+            dst[lane * 4 + i] = v;
+            nz = nz || v != 0.f;
           }
           // an all-zero bias (no padding in this key block) lets the softmax warps skip it
-          const bool nz = dst[lane * 4] != 0.f || dst[lane * 4 + 1] != 0.f || dst[lane * 4 + 2] != 0.f || dst[lane * 4 + 3] != 0.f;
           const bool any_nz = __any_sync(0xffffffffu, nz);
-          if (lane == 0) bars->bias_nz[kcount % kWsBiasRing] = any_nz ? 1 : 0;
+          if (lane == 0) bars->bias_nz[kcount % kFwdBiasRing] = any_nz ? 1 : 0;
           __threadfence_block();
         }
         __syncwarp();
         if (lane == 0) {
-          mbar_expect_tx(&bars->k_full[ks], kImg);
-          tma_load_4d(k_img + ks * kImg, &map_k, &bars->k_full[ks], 0, j * kBlk, h, b);
-          ok = mbar_wait_ol(&bars->v_empty, (vcount & 1) ^ 1, abort_flag, p.status, t);
+          mbar_expect_tx(&bars->kv_full[ks], kImg);
+          tma_tile<NB>(kv_img + ks * kImg, &map_k, &bars->kv_full[ks], j * kBlk, h, b);
+          const int vs = (kv + 1) % kFwdRing, vp = ((kv + 1) / kFwdRing) & 1;
+          ok = mbar_wait_ol(&bars->kv_empty[vs], vp ^ 1, abort_flag, p.status, t);
           if (ok) {
-            mbar_expect_tx(&bars->v_full, kImg);
-            tma_load_4d(v_img, &map_v, &bars->v_full, 0, j * kBlk, h, b);
+            mbar_expect_tx(&bars->kv_full[vs], kImg);
+            tma_tile<NB>(kv_img + vs * kImg, &map_v, &bars->kv_full[vs], j * kBlk, h, b);
           }
         }
-        ++kcount; ++vcount;
+        kv += 2; ++kcount;
       }
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
     }
   } else if (warp >= 8) {
-    // =========================================================================== MMA issuer of lane w
-    if (lane == 0) {
-      const uint32_t idesc_s = make_idesc_f16(kBlk, kBlk, false, false, p.is_bf16);
-      const uint32_t idesc_o = make_idesc_f16(kBlk, DP, false, true, p.is_bf16);
-      int kcount = 0, vcount = 0, pcount = 0, fcount = 0, tile_it = 0;
-      bool ok = true;
-      auto issue_s = [&](bool last) -> bool {
-        const int ks = kcount % kWsKRing;
-        if (!mbar_wait_ol(&bars->k_full[ks], (kcount / kWsKRing) & 1, abort_flag, p.status, kcount)) return false;
-        tc_fence_after();
+    // =========================================================================== MMA issuers
+    const uint32_t idesc_s = make_idesc_f16(kBlk, kBlk, false, false, p.is_bf16);
+    const uint32_t idesc_o = make_idesc_f16(kBlk, DP, false, true, p.is_bf16);
+    auto wait = [&](uint64_t* bar, int use, int detail) { return mbar_wait_ol(bar, use & 1, abort_flag, p.status, detail); };
+    // S_w from the K block in ring use `st`
+    auto issue_s = [&](int w, int st, bool last_use, bool last_block, int t) -> bool {
+      const int ks = st % kFwdRing;
+      if (!wait(&bars->kv_full[ks], st / kFwdRing, t)) return false;
+      tc_fence_after();
 #pragma unroll
-        for (int k16 = 0; k16 < DP / 16; ++k16)
-          tc_mma_f16(tm_s, kmajor_desc(smem_u32(q_img), k16), kmajor_desc(smem_u32(k_img + ks * kImg), k16), idesc_s, k16 > 0);
-        tc_commit(&bars->k_empty[ks]);
-        tc_commit(&bars->s_full);
-        if (last) tc_commit(&bars->q_empty);
-        ++kcount;
-        return true;
-      };
-      for (int t = first; t < tiles && ok && !*abort_flag; t += stride, ++tile_it) {
-        const int qb = n_qb - 1 - t / bh_total;
-        const int n_kv = n_kv_of(qb);
-        ok = mbar_wait_ol(&bars->q_full, tile_it & 1, abort_flag, p.status, t);
-        ok = ok && issue_s(n_kv == 1);
-        for (int j = 0; j < n_kv && ok; ++j) {
+      for (int k16 = 0; k16 < DP / 16; ++k16)
+        tc_mma_f16(tmem + w * 128, kmajor_desc(smem_u32(q_img + w * kImg), k16), kmajor_desc(smem_u32(kv_img + ks * kImg), k16),
+                   idesc_s, k16 > 0);
+      tc_commit(&bars->s_full[w]);
+      if (last_use) tc_commit(&bars->kv_empty[ks]);
+      if (last_block) tc_commit(&bars->q_empty[w]);
+      return true;
+    };
+    // O_w (+)= P_w V with the V block in ring use `st`, once the group has handed over P_w
+    auto issue_pv = [&](int w, int st, int p_use, bool first_block, bool last_use, int t) -> bool {
+      const int vs = st % kFwdRing;
+      if (!wait(&bars->p_ready[w], p_use, t) || !wait(&bars->kv_full[vs], st / kFwdRing, t)) return false;
+      const uint32_t tm_o = tmem + 256 + w * (kOwnP ? 64 : 128), tm_p = kOwnP ? tmem + 384 + w * 64 : tmem + w * 128;
+      tc_fence_after();
+#pragma unroll
+      for (int k16 = 0; k16 < kBlk / 16; ++k16)
+        tc_mma_f16_ts(tm_o, tm_p + k16 * 8, mnmajor_desc(smem_u32(kv_img + vs * kImg), k16), idesc_o,
+                      (!first_block || k16 > 0) ? 1u : 0u);
+      tc_commit(&bars->o_full[w]);
+      if (last_use) tc_commit(&bars->kv_empty[vs]);
+      return true;
+    };
+    int kv = 0;                                    // ring uses before this item
+    bool ok = true;
+    if (kOwnP && lane == 0) {
+      // one issuer per lane: neither waits for the other's group
+      const int w = warp - 8;
+      int q_use = 0, s_use = 0, p_use = 0;         // uses of q_full / of s_free / of p_ready and o_full
+      for (int t = first; t < items && ok && !*abort_flag; t += stride) {
+        const int qb0 = 2 * (n_pair - 1 - t / bh_total);
+        const int n = n_kv_of(qb0 + w), n_kv = max(n_kv_of(qb0), n_kv_of(qb0 + 1));
+        if (n > 0) ok = wait(&bars->q_full[w], q_use++, t) && issue_s(w, kv, true, n == 1, t);
+        for (int j = 0; j < n && ok; ++j) {
+          const int st = kv + 2 * j + 1;
           // the group has read S_j for the last time: S_{j+1} goes first, it is what the group needs soonest
-          ok = mbar_wait_ol(&bars->s_free, fcount & 1, abort_flag, p.status, t);
-          if (!ok) break;
-          ++fcount;
-          if (j + 1 < n_kv) {
+          ok = wait(&bars->s_free[w], s_use++, t);
+          if (ok && j + 1 < n) {
             tc_fence_after();
-            ok = issue_s(j + 1 == n_kv - 1);
-            if (!ok) break;
+            ok = issue_s(w, st + 1, true, j + 2 == n, t);
           }
-          ok = mbar_wait_ol(&bars->p_ready, pcount & 1, abort_flag, p.status, t);
-          if (!ok) break;
-          ++pcount;
-          ok = mbar_wait_ol(&bars->v_full, vcount & 1, abort_flag, p.status, t);
-          if (!ok) break;
-          tc_fence_after();
-#pragma unroll
-          for (int k16 = 0; k16 < kBlk / 16; ++k16)
-            tc_mma_f16(tm_o, kmajor_desc(smem_u32(p_img), k16), mnmajor_desc(smem_u32(v_img), k16), idesc_o,
-                       (j > 0 || k16 > 0) ? 1u : 0u);
-          tc_commit(&bars->v_empty);
-          tc_commit(&bars->o_full);
-          ++vcount;
+          ok = ok && issue_pv(w, st, p_use++, j == 0, true, t);
         }
+        // blocks that only the other lane uses: hand them back once they have arrived (earlier would count for an older use)
+        for (int st = kv + 2 * n; st < kv + 2 * n_kv && ok; ++st) {
+          ok = wait(&bars->kv_full[st % kFwdRing], st / kFwdRing, t);
+          if (ok) mbar_arrive(&bars->kv_empty[st % kFwdRing]);
+        }
+        kv += 2 * n_kv;
+      }
+    } else if (!kOwnP && warp == 8 && lane == 0) {
+      // one issuer for both lanes, in turn: that keeps them out of phase, one computing exponentials while the other's
+      // products run (with an issuer each they drift into step: 524 us instead of 379 for 4 x 40 heads x 2048 x 128)
+      int q_use[2] = {0, 0}, p_use[2] = {0, 0};
+      // the next scores lie over P: once P V has finished with it
+      auto next_s = [&](int w, int st, bool last_use, bool last_block, int t) {
+        return (p_use[w] == 0 || wait(&bars->o_full[w], p_use[w] - 1, t)) && issue_s(w, st, last_use, last_block, t);
+      };
+      for (int t = first; t < items && ok && !*abort_flag; t += stride) {
+        const int qb0 = 2 * (n_pair - 1 - t / bh_total);
+        const int n[2] = {n_kv_of(qb0), n_kv_of(qb0 + 1)};
+        const int n_kv = max(n[0], n[1]);
+        const int last = n[1] > 0 ? 1 : 0;         // the lane that uses every key block, and after the other one
+#pragma unroll
+        for (int w = 0; w < 2; ++w)
+          if (ok && n[w] > 0) ok = wait(&bars->q_full[w], q_use[w]++, t) && next_s(w, kv, w == last, n[w] == 1, t);
+        for (int j = 0; j < n_kv && ok; ++j) {
+          const int st = kv + 2 * j + 1;
+#pragma unroll
+          for (int w = 0; w < 2; ++w) {
+            if (!ok || j >= n[w]) continue;
+            ok = issue_pv(w, st, p_use[w]++, j == 0, w == last, t);
+            if (ok && j + 1 < n[w]) ok = next_s(w, st + 1, w == last, j + 2 == n[w], t);
+          }
+        }
+        kv += 2 * n_kv;
       }
     }
   } else {
     // =========================================================================== softmax group of lane w
+    const int w = warp >> 2;
     const int r = threadIdx.x & 127;                 // query row inside the tile == TMEM lane
     const int wq = warp & 3;                         // this warp's 32-row block
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
+    const uint32_t s_addr = tmem + w * 128 + lane_base, o_addr = tmem + 256 + w * (kOwnP ? 64 : 128) + lane_base;
+    const uint32_t p_addr = kOwnP ? tmem + 384 + w * 64 + lane_base : s_addr;
     const float sc2 = p.scale * kLog2e;
-    int scount = 0, ocount = 0, kbase = 0;           // uses of s_full / o_full; key blocks before this tile
+    int use = 0, kbase = 0;                          // uses of s_full / o_full; key blocks before this item
     bool ok = true;
     int ntr = 0;
-    long long* tr = threadIdx.x == 0 ? p.trace : nullptr;
-    for (int t = first; t < tiles && ok; t += stride) {
-      const int qb = n_qb - 1 - t / bh_total, bh = t % bh_total;
+    auto stamp = [&](int code) {                     // (kept out of the instantiations that are short of registers)
+      if constexpr (kOwnP) attn_trace(threadIdx.x == 0 ? p.trace : nullptr, 0, ntr, code);
+    };
+    for (int t = first; t < items && ok; t += stride) {
+      const int qb0 = 2 * (n_pair - 1 - t / bh_total), bh = t % bh_total;
       const int h = bh % p.H, b = bh / p.H;
-      const int n_kv = n_kv_of(qb);
+      const int qb = qb0 + w, n_kv = n_kv_of(qb);
+      const int item_kv = max(n_kv_of(qb0), n_kv_of(qb0 + 1));
       const int q_idx = qb * kBlk + r;
       float m_run = -INFINITY, l_run = 0.f;
       for (int j = 0; j < n_kv; ++j) {
         const int k0 = j * kBlk;
-        attn_trace(tr, 0, ntr, 1);
-        if (!mbar_wait_ol(&bars->s_full, scount & 1, abort_flag, p.status, t)) { ok = false; break; }
-        ++scount;
+        stamp(1);
+        if (!mbar_wait_ol(&bars->s_full[w], use & 1, abort_flag, p.status, t)) { ok = false; break; }
         tc_fence_after();
-        attn_trace(tr, 0, ntr, 2);
+        stamp(2);
         const bool tail = k0 + kBlk > p.T;
         const bool cdiag = p.causal && j == qb;
-        const float* bias_j = s_bias + ((kbase + j) % kWsBiasRing) * kBlk;
-        const bool has_bias = p.key_bias != nullptr && bars->bias_nz[(kbase + j) % kWsBiasRing] != 0;
-        const uint32_t s_addr = tm_s + lane_base;
-        uint32_t ra[32], rb[32];
+        const bool plain = !tail && !cdiag;
+        const float* bias_j = s_bias + ((kbase + j) % kFwdBiasRing) * kBlk;
+        const bool has_bias = p.key_bias != nullptr && bars->bias_nz[(kbase + j) % kFwdBiasRing] != 0;
         float m_blk = -INFINITY;
-        // ---- pass 1: the row maximum.  The next chunk's TMEM load is in flight while the current one is reduced.
-        if (!tail && !cdiag) {
+        uint32_t ra[32], rb[32];
+        // ---- pass 1: the row maximum
+        if (plain) {
           // all four chunk loads are issued before the first is used: one TMEM round trip for the pass
           uint32_t rc[32], rd[32];
           tmem_ld_32x32(s_addr, ra);
@@ -609,83 +441,81 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           tmem_wait_ld_for(rb);
           tmem_wait_ld_for(rc);
           tmem_wait_ld_for(rd);
-#define CW_MAX_STEP(CUR, C)                                                                                   \
-          m_blk = has_bias ? chunk_max<false, true>(CUR, bias_j + (C) * 32, sc2, 0, 0, 0, false, m_blk)        \
-                           : chunk_max<false, false>(CUR, nullptr, sc2, 0, 0, 0, false, m_blk);
-          CW_MAX_STEP(ra, 0)
-          CW_MAX_STEP(rb, 1)
-          CW_MAX_STEP(rc, 2)
-          CW_MAX_STEP(rd, 3)
-#undef CW_MAX_STEP
+          if (has_bias) {
+            m_blk = chunk_max<false, true>(ra, bias_j, sc2, 0, 0, 0, false, m_blk);
+            m_blk = chunk_max<false, true>(rb, bias_j + 32, sc2, 0, 0, 0, false, m_blk);
+            m_blk = chunk_max<false, true>(rc, bias_j + 64, sc2, 0, 0, 0, false, m_blk);
+            m_blk = chunk_max<false, true>(rd, bias_j + 96, sc2, 0, 0, 0, false, m_blk);
+          } else {
+            m_blk = chunk_max<false, false>(ra, nullptr, sc2, 0, 0, 0, false, m_blk);
+            m_blk = chunk_max<false, false>(rb, nullptr, sc2, 0, 0, 0, false, m_blk);
+            m_blk = chunk_max<false, false>(rc, nullptr, sc2, 0, 0, 0, false, m_blk);
+            m_blk = chunk_max<false, false>(rd, nullptr, sc2, 0, 0, 0, false, m_blk);
+          }
         } else {
-          // diagonal block of a causal mask: chunks left of this warp's rows are plain, the chunk on the diagonal is
-          // tested key by key, chunks to the right contribute nothing.  A sequence tail is tested everywhere.
+          // the causal diagonal: chunks left of this warp's rows are plain, the one on the diagonal is tested key by key,
+          // those to the right contribute nothing.  A sequence tail is tested everywhere.
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
             if (!tail && c > wq) break;
             tmem_ld_32x32(s_addr + c * 32, ra);
             tmem_wait_ld_for(ra);
-            if (!tail && c < wq)
-              m_blk = has_bias ? chunk_max<false, true>(ra, bias_j + c * 32, sc2, 0, 0, 0, false, m_blk)
-                               : chunk_max<false, false>(ra, nullptr, sc2, 0, 0, 0, false, m_blk);
-            else
-              m_blk = has_bias ? chunk_max<true, true>(ra, bias_j + c * 32, sc2, k0 + c * 32, q_idx, p.T, cdiag, m_blk)
-                               : chunk_max<true, false>(ra, nullptr, sc2, k0 + c * 32, q_idx, p.T, cdiag, m_blk);
+            m_blk = has_bias ? chunk_max<true, true>(ra, bias_j + c * 32, sc2, k0 + c * 32, q_idx, p.T, cdiag, m_blk)
+                             : chunk_max<true, false>(ra, nullptr, sc2, k0 + c * 32, q_idx, p.T, cdiag, m_blk);
           }
         }
         if (!has_bias) m_blk *= sc2;                  // scale > 0: the maximum commutes with the scaling
-        attn_trace(tr, 0, ntr, 3);
-        const float m_new = fmaxf(m_run, m_blk);
-        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-        const float alpha = (m_run == -INFINITY) ? 0.f : ex2_approx(m_run - m_use);
-        m_run = m_new;
-        if (j > 0) {
-          // the previous P V has landed in O: rescale it in place before more is added
-          if (!mbar_wait_ol(&bars->o_full, ocount & 1, abort_flag, p.status, t)) { ok = false; break; }
-          ++ocount;
+        stamp(3);
+        // P_{j-1} V has landed: O is complete and P may be written again.  (Scores that share their columns with P were
+        // issued after that.)
+        if (kOwnP && j > 0) {
+          if (!mbar_wait_ol(&bars->o_full[w], (use - 1) & 1, abort_flag, p.status, t)) { ok = false; break; }
           tc_fence_after();
-          attn_trace(tr, 0, ntr, 4);
-          if (__any_sync(0xffffffffu, alpha != 1.f)) {
+        }
+        stamp(4);
+        const bool grow = m_blk > m_run + kRescaleLog2;      // also the first finite maximum
+        if (__any_sync(0xffffffffu, grow)) {
+          const float alpha = grow ? ((m_run == -INFINITY) ? 0.f : ex2_approx(m_run - m_blk)) : 1.f;
+          if (grow) m_run = m_blk;
+          l_run *= alpha;
+          if (j > 0) {
 #pragma unroll
             for (int c = 0; c < DP / 32; ++c) {
               uint32_t raw[32];
-              tmem_ld_32x32(tm_o + lane_base + c * 32, raw);
+              tmem_ld_32x32(o_addr + c * 32, raw);
               tmem_wait_ld_for(raw);
 #pragma unroll
               for (int i = 0; i < 32; ++i) raw[i] = __float_as_uint(__uint_as_float(raw[i]) * alpha);
-              tmem_st_32x32(tm_o + lane_base + c * 32, raw);
+              tmem_st_32x32(o_addr + c * 32, raw);
             }
-            tmem_wait_st();
           }
         }
-        // ---- pass 2: exponentials, P to shared memory
+        const float m_use = (m_run == -INFINITY) ? 0.f : m_run;
+        stamp(5);
+        // ---- pass 2: exponentials.  Where P shares the columns, chunk c's 16 columns of it lie below chunk c + 1's scores,
+        // which have been read by then.
         float l_blk = 0.f;
-        attn_trace(tr, 0, ntr, 5);
-        if (!tail && !cdiag) {
-          // chunks 0 and 1 are requested together; chunk c + 2 is requested before chunk c is processed
-          uint32_t rc[32];
+        if (plain) {
           tmem_ld_32x32(s_addr, ra);
-          tmem_ld_32x32(s_addr + 32, rb);
           tmem_wait_ld_for(ra);
-          tmem_wait_ld_for(rb);
-#define CW_EXP_STEP(CUR, C)                                                                                   \
-          {                                                                                                    \
-            float pv[32];                                                                                      \
-            l_blk += has_bias ? chunk_exp<false, true>(CUR, bias_j + (C) * 32, sc2, m_use, 0, 0, 0, false, pv) \
-                              : chunk_exp<false, false>(CUR, nullptr, sc2, m_use, 0, 0, 0, false, pv);         \
-            store_p_chunk<T>(p_img, r, (C) * 32, pv);                                                          \
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t(&cur)[32] = (c & 1) ? rb : ra;
+            uint32_t(&nxt)[32] = (c & 1) ? ra : rb;
+            if (c < 3) tmem_ld_32x32(s_addr + (c + 1) * 32, nxt);
+            float pv[32];
+            l_blk += has_bias ? chunk_exp<false, true>(cur, bias_j + c * 32, sc2, m_use, 0, 0, 0, false, pv)
+                              : chunk_exp<false, false>(cur, nullptr, sc2, m_use, 0, 0, 0, false, pv);
+            uint32_t pk[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) pk[i] = pack_pair<T>(pv[2 * i], pv[2 * i + 1]);
+            if (c < 3) tmem_wait_ld_for(nxt);
+            if (kOwnP && c == 2) {
+              tc_fence_before();
+              mbar_arrive(&bars->s_free[w]);          // last read of the scores: the next block's may overwrite them
+            }
+            tmem_st_32x16(p_addr + c * 16, pk);
           }
-          tmem_ld_32x32(s_addr + 64, rc);
-          CW_EXP_STEP(ra, 0)
-          tmem_wait_ld_for(rc);
-          tmem_ld_32x32(s_addr + 96, ra);
-          CW_EXP_STEP(rb, 1)
-          tmem_wait_ld_for(ra);
-          tc_fence_before();
-          mbar_arrive(&bars->s_free);                 // last read of the scores: the next block's S may overwrite them
-          CW_EXP_STEP(rc, 2)
-          CW_EXP_STEP(ra, 3)
-#undef CW_EXP_STEP
         } else {
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
@@ -696,42 +526,46 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             } else {
               tmem_ld_32x32(s_addr + c * 32, ra);
               tmem_wait_ld_for(ra);
-              if (!tail && c < wq)
-                l_blk += has_bias ? chunk_exp<false, true>(ra, bias_j + c * 32, sc2, m_use, 0, 0, 0, false, pv)
-                                  : chunk_exp<false, false>(ra, nullptr, sc2, m_use, 0, 0, 0, false, pv);
-              else
-                l_blk += has_bias ? chunk_exp<true, true>(ra, bias_j + c * 32, sc2, m_use, k0 + c * 32, q_idx, p.T, cdiag, pv)
-                                  : chunk_exp<true, false>(ra, nullptr, sc2, m_use, k0 + c * 32, q_idx, p.T, cdiag, pv);
+              l_blk += has_bias ? chunk_exp<true, true>(ra, bias_j + c * 32, sc2, m_use, k0 + c * 32, q_idx, p.T, cdiag, pv)
+                                : chunk_exp<true, false>(ra, nullptr, sc2, m_use, k0 + c * 32, q_idx, p.T, cdiag, pv);
             }
-            store_p_chunk<T>(p_img, r, c * 32, pv);
+            uint32_t pk[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) pk[i] = pack_pair<T>(pv[2 * i], pv[2 * i + 1]);
+            tmem_st_32x16(p_addr + c * 16, pk);
           }
-          tc_fence_before();
-          mbar_arrive(&bars->s_free);
+          if (kOwnP) {
+            tc_fence_before();
+            mbar_arrive(&bars->s_free[w]);
+          }
         }
-        l_run = l_run * alpha + l_blk;
-        attn_trace(tr, 0, ntr, 6);
-        fence_proxy_async();
+        l_run += l_blk;
+        stamp(6);
+        tmem_wait_st();
         tc_fence_before();
-        mbar_arrive(&bars->p_ready);
-        attn_trace(tr, 0, ntr, 7);
+        mbar_arrive(&bars->p_ready[w]);
+        stamp(7);
+        ++use;
       }
       if (!ok) break;
+      kbase += item_kv;
+      if (n_kv == 0) continue;
       // ---- the tile's output: the last P V has landed
-      if (!mbar_wait_ol(&bars->o_full, ocount & 1, abort_flag, p.status, t)) { ok = false; break; }
-      ++ocount;
+      if (!mbar_wait_ol(&bars->o_full[w], (use - 1) & 1, abort_flag, p.status, t)) { ok = false; break; }
       tc_fence_after();
-      attn_trace(tr, 0, ntr, 8);
-      {
-        // rows go through shared memory (the P image is free now) so that each global store instruction writes one
-        // row's contiguous bytes instead of one column of 32 rows that lie kilobytes apart
-        const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-        T* stage = reinterpret_cast<T*>(p_img) + wq * 32 * DP;          // this warp's [32][DP]
+      stamp(8);
+      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+      const int64_t row_pitch = static_cast<int64_t>(p.H) * p.dh;
+      const int row0 = qb * kBlk + wq * 32;
+      T* o = reinterpret_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.T + row0) * row_pitch + static_cast<int64_t>(h) * p.dh;
+      const bool vec = p.dh % 8 == 0;                // rows start on 16-byte boundaries
+      T* stage = reinterpret_cast<T*>(out_stage) + (warp * 32 + lane) * (kOwnP ? DP : 0);
 #pragma unroll
-        for (int c = 0; c < DP / 32; ++c) {
-          uint32_t raw[32];
-          tmem_ld_32x32(tm_o + lane_base + c * 32, raw);
-          tmem_wait_ld_for(raw);
-          uint4* dst = reinterpret_cast<uint4*>(stage + lane * DP + c * 32);
+      for (int c = 0; c < DP / 32; ++c) {
+        uint32_t raw[32];
+        tmem_ld_32x32(o_addr + c * 32, raw);
+        tmem_wait_ld_for(raw);
+        if (vec || kOwnP) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             uint4 u;
@@ -739,22 +573,32 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             u.y = pack_pair<T>(__uint_as_float(raw[q * 8 + 2]) * inv, __uint_as_float(raw[q * 8 + 3]) * inv);
             u.z = pack_pair<T>(__uint_as_float(raw[q * 8 + 4]) * inv, __uint_as_float(raw[q * 8 + 5]) * inv);
             u.w = pack_pair<T>(__uint_as_float(raw[q * 8 + 6]) * inv, __uint_as_float(raw[q * 8 + 7]) * inv);
-            dst[q] = u;
+            if (!vec) {
+              *reinterpret_cast<uint4*>(stage + c * 32 + q * 8) = u;
+            } else if (q_idx < p.T && c * 32 + q * 8 < p.dh) {
+              *reinterpret_cast<uint4*>(o + lane * row_pitch + c * 32 + q * 8) = u;
+            }
           }
+        } else if (q_idx < p.T) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i < p.dh) o[lane * row_pitch + c * 32 + i] = from_f<T>(__uint_as_float(raw[i]) * inv);
         }
-        if (q_idx < p.T)
-          p.lse[(static_cast<int64_t>(b) * p.H + h) * p.T + q_idx] = (l_run > 0.f) ? m_run + log2f(l_run) : -INFINITY;
-        tc_fence_before();
+      }
+      if (q_idx < p.T)
+        p.lse[(static_cast<int64_t>(b) * p.H + h) * p.T + q_idx] = (l_run > 0.f) ? m_run + log2f(l_run) : -INFINITY;
+      tc_fence_before();                             // ordered before the group's next hand-over, which lets O be overwritten
+      if (kOwnP && !vec) {
+        // rows go through shared memory so that each global store instruction writes one row's contiguous bytes instead of
+        // one column of 32 rows that lie kilobytes apart
         __syncwarp();
-        const int row0 = qb * kBlk + wq * 32;
-        T* o = reinterpret_cast<T*>(p.out) + ((static_cast<int64_t>(b) * p.T + row0) * p.H + h) * p.dh;
-        const int64_t row_pitch = static_cast<int64_t>(p.H) * p.dh;
+        const T* rows_in = reinterpret_cast<const T*>(out_stage) + warp * 32 * DP;
         const int rows = min(32, p.T - row0);
         for (int d = lane; d < p.dh; d += 32) {
           for (int r0 = 0; r0 < rows; r0 += 8) {
             T v[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = stage[min(r0 + u, 31) * DP + d];
+            for (int u = 0; u < 8; ++u) v[u] = rows_in[min(r0 + u, 31) * DP + d];
 #pragma unroll
             for (int u = 0; u < 8; ++u)
               if (r0 + u < rows) o[(r0 + u) * row_pitch + d] = v[u];
@@ -762,8 +606,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
         __syncwarp();
       }
-      attn_trace(tr, 0, ntr, 9);
-      kbase += n_kv;
+      stamp(9);
     }
     if (!ok) *abort_flag = 1;
   }
@@ -1850,8 +1693,6 @@ static int padded_dim(int dh) {
   return dh <= 32 ? 32 : dh <= 64 ? 64 : dh <= 96 ? 96 : 128;
 }
 template <int DP>
-constexpr int fwd_smem() { return 3 * ((DP + 63) / 64) * kBlk * 128 + 2 * kBlk * 128 + 64 + 1024 + 1024; }
-template <int DP>
 constexpr int bwd_smem() {
   return (DP <= 64 ? 6 : 4) * ((DP + 63) / 64) * kBlk * 128 + 4 * kBlk * 128 + 64 + 1024 + 512 +
          (DP <= 64 ? kBlk * DP * 4 : 0);
@@ -1863,33 +1704,16 @@ struct AttnMaps {
 };
 
 template <typename T, int DP>
-static void launch_fwd_ws(const AttnMaps& m, const AttnParams& p, cudaStream_t s) {
-  auto kern = attn_fwd_ws_kernel<T, DP>;
-  static bool done = false;
-  if (!done) {
-    C10_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_ws_smem<DP>()));
-    done = true;
-  }
-  const int tiles = ((p.T + kBlk - 1) / kBlk) * p.H * p.B;
-  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  kern<<<std::min(tiles, sms), kWsThreads, fwd_ws_smem<DP>(), s>>>(m.q, m.k, m.v, p);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
-}
-
-template <typename T, int DP>
 static void launch_fwd(const AttnMaps& m, const AttnParams& p, cudaStream_t s) {
-  if constexpr (DP <= 64) {
-    launch_fwd_ws<T, DP>(m, p, s);
-    return;
-  }
   auto kern = attn_fwd_kernel<T, DP>;
   static bool done = false;
   if (!done) {
     C10_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_smem<DP>()));
     done = true;
   }
-  dim3 grid((p.T + kBlk - 1) / kBlk, p.H, p.B);
-  kern<<<grid, kAttnThreads, fwd_smem<DP>(), s>>>(m.q, m.k, m.v, p);
+  const int items = ((p.T + 2 * kBlk - 1) / (2 * kBlk)) * p.H * p.B;
+  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  kern<<<std::min(items, sms), kFwdThreads, fwd_smem<DP>(), s>>>(m.q, m.k, m.v, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 template <typename T, int DP>

@@ -63,6 +63,42 @@ def test_wide_layer_norm_with_residual(rows, H, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,H,dh,causal,pad", [
+    (1, 1, 1, 80, True, False),          # one row of one tile
+    (1, 128, 3, 128, True, False),       # one full tile, its neighbour does not exist
+    (2, 129, 2, 128, True, True),        # one row in the second tile
+    (1, 257, 4, 72, False, False),       # an odd number of tiles, no mask
+    (2, 640, 5, 96, True, True),         # more key blocks than ring stages
+    (3, 300, 2, 100, True, False),       # a head dim that needs the padded copy
+    (2, 197, 3, 48, False, False),       # the vector row sums with idle lanes
+    (2, 70, 3, 24, True, False),         # ... and with four lanes
+    (4, 900, 40, 128, True, True),       # several items per CTA
+])
+def test_attention_tiles(dtype, B, T, H, dh, causal, pad):
+    ops, ext = _ops()
+    g = torch.Generator(device="cuda").manual_seed(B * T + dh)
+    qkv = torch.randn(B, T, H, 3 * dh, generator=g, device="cuda")
+    qkv[..., :dh] *= 3.0                                          # scores that make the running maximum move
+    qkv = qkv.to(dtype).requires_grad_(True)
+    bias = None
+    if pad:
+        bias = torch.zeros(B, T, device="cuda")
+        bias[-1, T // 2:] = -10000.0
+    dout = torch.randn(B, T, H * dh, generator=g, device="cuda").to(dtype)
+    out = ops.attention_packed(qkv, causal, bias)
+    out.backward(dout)
+    ext.check_status()
+    ref_in = qkv.detach().float().requires_grad_(True)
+    q, k, v = ref_in.permute(0, 2, 1, 3).chunk(3, dim=-1)
+    ref = ops.attention_reference(q, k, v, causal, bias).transpose(1, 2).reshape(B, T, H * dh)
+    ref.backward(dout.float())
+    # probabilities and results rounded to 16 bits; gradients pass two such products more
+    tol = 4 * UNIT[dtype]
+    assert (out.float() - ref).norm() <= tol * ref.norm()
+    assert (qkv.grad.float() - ref_in.grad).norm() <= 2 * tol * ref_in.grad.norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("trans_a,trans_b", [(False, True), (False, False), (True, False), (True, True)])
 @pytest.mark.parametrize("M,N,K", [
     (256, 256, 64),            # one tile, one k-block
