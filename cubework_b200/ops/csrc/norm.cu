@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kNT) row_moments_kernel(const T* __restrict__ 
 // are converted twice; the next row is requested into L2 meanwhile.  8192 x 5120: 181 -> 83 us, 117 with the residual's
 // gradient (336 MB; 205 while it was left at one CTA per SM by its registers).
 template <typename T, int MODE, int VPT, bool HAS_RES>
-__global__ void __launch_bounds__(kNT, VPT <= 3 ? 2 : 1) ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
+__global__ void __launch_bounds__(kNT, VPT == 1 ? 4 : VPT <= 3 ? 2 : 1) ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                                                      const float* __restrict__ mean, const float* __restrict__ rstd,
                                                      const float* __restrict__ gamma, const T* __restrict__ dres,
                                                      T* __restrict__ dx, float* __restrict__ row_sums,
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(kNT, VPT <= 3 ? 2 : 1) ln_bwd_kernel(const T* 
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Warp-per-row layer norm for hidden sizes up to 2048: a row lives in one warp's registers (NV 16-byte vectors
+// Warp-per-row layer norm for hidden sizes up to 2048 (backward: up to 1280): a row lives in one warp's registers (NV 16-byte vectors
 // per lane), the two statistics are warp shuffles, and nothing synchronises the CTA, so eight rows per CTA are in
 // flight with all their loads outstanding.  Optionally fused with the residual add in front of the norm
 // (reference: `x = x + dropout(...)` followed by `norm(x)`, benchmark/gpt2/gpt2.py:179-186): forward writes the sum
@@ -644,9 +644,10 @@ static void ln_bwd_launch(const torch::Tensor& dy, const torch::Tensor& x, const
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 
-static int bwd_grid(int rows) {
+// persistent over rows: as many CTAs as are resident at once
+static int bwd_grid(int rows, int H) {
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  return std::max(1, std::min(rows, sms * 2));
+  return std::max(1, std::min(rows, sms * (H <= kNT * 8 ? 4 : 2)));
 }
 
 static std::vector<torch::Tensor> layer_norm_bwd_cta(torch::Tensor dy, torch::Tensor x, torch::Tensor mean, torch::Tensor rstd,
@@ -659,7 +660,7 @@ static std::vector<torch::Tensor> layer_norm_bwd_cta(torch::Tensor dy, torch::Te
   auto f32 = x.options().dtype(torch::kFloat32);
   if (rows == 0) return {dx, torch::zeros({H}, f32), torch::zeros({H}, f32)};
   auto dgamma = torch::empty({H}, f32), dbeta = torch::empty({H}, f32);
-  const int grid = bwd_grid(rows);
+  const int grid = bwd_grid(rows, H);
   auto scratch = torch::empty({2, grid, H}, f32);
   auto stream = at::cuda::getCurrentCUDAStream();
   float* pdg = scratch.data_ptr<float>();
@@ -686,7 +687,7 @@ std::vector<torch::Tensor> norm_bwd_partials(torch::Tensor dy, torch::Tensor x, 
   if (rows == 0) return {sums, torch::zeros({H}, f32), torch::zeros({H}, f32)};
   gamma = aligned16(gamma);
   auto dgamma = torch::empty({H}, f32), dbeta = torch::empty({H}, f32);
-  const int grid = bwd_grid(rows);
+  const int grid = bwd_grid(rows, H);
   auto scratch = torch::empty({2, grid, H}, f32);
   auto stream = at::cuda::getCurrentCUDAStream();
   float* pdg = scratch.data_ptr<float>();
@@ -732,6 +733,27 @@ constexpr int kWarpMaxH = 2048;
     DISPATCH_NV((x).size(1), __VA_ARGS__)                          \
   }
 
+// The backward of rows above 1280 columns takes a CTA per row, four per SM, with the parameter gradients in registers: by
+// warps, sixteen rows per SM wait for their loads (32768 x 1600 with a residual 163 us, 120 by CTAs; 4096 x 2048 56 and 32;
+// at 1280 65 and 60, without a residual 52 and 54; at 768 99 and 136).
+constexpr int kWarpMaxBwd = 1280;
+#define DISPATCH_16_NV_BWD(x, ...)                                 \
+  {                                                                \
+    const int need_ = ((x).size(1) / 8 + 31) / 32;                 \
+    if ((x).scalar_type() == torch::kBFloat16) {                   \
+      using T = __nv_bfloat16;                                     \
+      DISPATCH_NV_BWD(__VA_ARGS__)                                 \
+    } else {                                                       \
+      using T = __half;                                            \
+      DISPATCH_NV_BWD(__VA_ARGS__)                                 \
+    }                                                              \
+  }
+#define DISPATCH_NV_BWD(...)                                       \
+  if (need_ <= 1) { constexpr int NV = 1; __VA_ARGS__ }            \
+  else if (need_ <= 2) { constexpr int NV = 2; __VA_ARGS__ }       \
+  else if (need_ <= 4) { constexpr int NV = 4; __VA_ARGS__ }       \
+  else { constexpr int NV = 5; __VA_ARGS__ }
+
 static bool warp_path(const torch::Tensor& x) { return x.size(1) <= kWarpMaxH; }
 
 // y = LN(x (+ residual)); returns {y, mean, rstd, sum}: `sum` is x + residual (undefined without a residual).
@@ -743,9 +765,10 @@ std::vector<torch::Tensor> layer_norm_fwd_res(torch::Tensor x, c10::optional<tor
   TORCH_CHECK((gamma.scalar_type() == torch::kFloat32 || gamma.scalar_type() == x.scalar_type()) &&
               beta.scalar_type() == gamma.scalar_type() && gamma.is_contiguous() && beta.is_contiguous() &&
               gamma.numel() == H && beta.numel() == H, "norm parameters must be contiguous [H], fp32 or of the rows' type");
-  // A CTA per row for wide rows, and for so few that eight rows per CTA leave most SMs without one (decoding: 8 rows of 2048
+  // A CTA per row for wide rows (with a residual from 1536 columns on: 32768 x 1600 104 us by warps, 96 by CTAs, 4096 x 2048 28
+  // and 21; without one the warps stay ahead at 1600, 52 and 76), and for so few that eight rows per CTA leave most SMs without one (decoding: 8 rows of 2048
   // took 9.2 us on one SM, every vector of a row in the same 32 lanes; 2.4 us now).
-  const bool cta = !warp_path(x) || rows <= 2 * at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  const bool cta = !warp_path(x) || (has_res && H > 1536) || rows <= 2 * at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   torch::Tensor sum;
   if (has_res) {
     check_rows(*residual);
@@ -790,7 +813,7 @@ std::vector<torch::Tensor> layer_norm_bwd_res(torch::Tensor dy, torch::Tensor x,
     check_rows(*dres);
     TORCH_CHECK(dres->sizes() == x.sizes() && dres->scalar_type() == x.scalar_type());
   }
-  if (!warp_path(x)) return layer_norm_bwd_cta(dy, x, mean, rstd, gamma, has_res ? &*dres : nullptr);
+  if (x.size(1) > kWarpMaxBwd) return layer_norm_bwd_cta(dy, x, mean, rstd, gamma, has_res ? &*dres : nullptr);
   const int rows = x.size(0), H = x.size(1);
   TORCH_CHECK(gamma.scalar_type() == torch::kFloat32 && gamma.is_contiguous() && gamma.numel() == H);
   gamma = aligned16(gamma);
@@ -806,11 +829,11 @@ std::vector<torch::Tensor> layer_norm_bwd_res(torch::Tensor dy, torch::Tensor x,
   float* pdb = pdg + static_cast<size_t>(grid) * H;
   const size_t smem = static_cast<size_t>(kWarpRows) * 2 * H * sizeof(float);
   if (has_res) {
-    DISPATCH_16_NV(x, (launch_ln_bwd_warp<T, NV, true>(grid, smem, stream, dy.data_ptr(), x.data_ptr(), mean.data_ptr<float>(),
+    DISPATCH_16_NV_BWD(x, (launch_ln_bwd_warp<T, NV, true>(grid, smem, stream, dy.data_ptr(), x.data_ptr(), mean.data_ptr<float>(),
                                                        rstd.data_ptr<float>(), gamma.data_ptr<float>(), dres->data_ptr(),
                                                        dx.data_ptr(), pdg, pdb, rows, H));)
   } else {
-    DISPATCH_16_NV(x, (launch_ln_bwd_warp<T, NV, false>(grid, smem, stream, dy.data_ptr(), x.data_ptr(), mean.data_ptr<float>(),
+    DISPATCH_16_NV_BWD(x, (launch_ln_bwd_warp<T, NV, false>(grid, smem, stream, dy.data_ptr(), x.data_ptr(), mean.data_ptr<float>(),
                                                         rstd.data_ptr<float>(), gamma.data_ptr<float>(), nullptr, dx.data_ptr(),
                                                         pdg, pdb, rows, H));)
   }

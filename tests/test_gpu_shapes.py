@@ -38,7 +38,8 @@ def test_act_backward_stripes(M, N, act):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("rows,H", [(1, 2056), (300, 4096), (1200, 5120), (5, 6144), (7, 8200), (3, 16384)])
+@pytest.mark.parametrize("rows,H", [(1, 8), (1, 2056), (300, 4096), (1200, 5120), (5, 6144), (7, 8200), (3, 16384),
+                                    (700, 1280), (297, 1288), (700, 1536), (700, 1544), (2000, 2048)])   # ends of the rules
 def test_wide_layer_norm_with_residual(rows, H, dtype):
     ops, _ = _ops()
     g = torch.Generator(device="cuda").manual_seed(rows + H)
@@ -58,8 +59,8 @@ def test_wide_layer_norm_with_residual(rows, H, dtype):
     # fp32 sums over the rows of terms below 36
     bound = rows * 2.0**-24 * 36 * rows + 1e-4
     assert ((dg.double() - gd.grad).abs() <= bound).all() and ((db.double() - bd.grad).abs() <= bound).all()
-    y2, _, _ = ops.layer_norm_fwd(total, gamma, beta, 1e-5)
-    assert torch.equal(y2, y)
+    y2, _, _ = ops.layer_norm_fwd(total, gamma, beta, 1e-5)       # may sum in another order (another kernel)
+    assert ((y2.double() - ref).abs() <= UNIT[dtype] * ref.abs() + 1e-5).all()
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
