@@ -101,10 +101,16 @@ def _register_shadow_finalizer(param, key):
 _ACT_CODE = {None: 0, "gelu": 1, "relu": 2}
 
 
+def _recorded() -> bool:
+    """A call made while ``torch.jit.trace`` records or under a function transform.  A trace takes a Python function as one
+    opaque node, but goes through a native one operator by operator: it would keep the allocation of the result and not the
+    kernel that fills it.  Transforms refuse the Python functions and would not see the native ones."""
+    return torch._C._get_tracing_state() is not None or torch._C._are_functorch_transforms_active()
+
+
 def _native(x, cd) -> bool:
-    """The native nodes take CUDA tensors with a 16-bit compute dtype, outside function transforms (which refuse the Python
-    functions and would not see the native ones)."""
-    if not (x.is_cuda and cd in _LOWP and kernels_enabled()) or torch._C._are_functorch_transforms_active():
+    """The native nodes take CUDA tensors with a 16-bit compute dtype, in calls that nothing records."""
+    if not (x.is_cuda and cd in _LOWP and kernels_enabled()) or _recorded():
         return False
     ext.require()
     return True
@@ -384,8 +390,11 @@ def _needs_grad(*tensors):
 
 def decode_ready(qkv, k_past, v_past, key_bias) -> bool:
     """Whether :func:`decode_attention` takes these tensors: one query token, no gradients, 16-bit caches of the
-    projection's dtype with dense 16-byte aligned rows, one bias value per key.  Everything else (several query tokens
-    against a cache, mixed dtypes, head dims that are no multiple of 8) keeps the materialised formulation."""
+    projection's dtype with dense 16-byte aligned rows, one bias value per key, nothing that records the call.
+    Everything else (several query tokens against a cache, mixed dtypes, head dims that are no multiple of 8) keeps the
+    materialised formulation."""
+    if _recorded():
+        return False
     B, T, H, D3 = qkv.shape
     dh = D3 // 3
     if T != 1 or dh % 8 or dh > 256 or not use_kernels(qkv) or not qkv.is_contiguous() or qkv.data_ptr() % 16:
@@ -413,9 +422,9 @@ def decode_attention(qkv, k_past, v_past, key_bias=None, scale=None):
 def prefill_ready(qkv, key_bias) -> bool:
     """Whether a cached prompt may run through :func:`attention_packed`: no gradients, and 16-bit autocast, under which
     the materialised formulation rounds its scores and probabilities to 16 bits as well (without autocast it keeps
-    them in fp32, and so does this framework)."""
+    them in fp32, and so does this framework).  A recorded call keeps the formulation's operators."""
     B, T, H, D3 = qkv.shape
-    return (use_kernels(qkv) and D3 // 3 <= 128 and torch.is_autocast_enabled("cuda")
+    return (not _recorded() and use_kernels(qkv) and D3 // 3 <= 128 and torch.is_autocast_enabled("cuda")
             and torch.get_autocast_dtype("cuda") in _LOWP
             and (key_bias is None or (key_bias.device == qkv.device and tuple(key_bias.shape) == (B, T)))
             and not _needs_grad(qkv, key_bias))
