@@ -142,8 +142,9 @@ class Trainer:
 
     def _folds_clipping(self):
         """The clipping factor may go into the optimizer's own pass over the gradients: a fused optimizer with its own
-        ``step`` that updates every parameter with a gradient (clipping scales each of them), no loss scaler between, and
-        no hook that could look at the gradients in between."""
+        ``step`` that updates the model's parameters with a gradient and no others (clipping scales each of the former, and
+        the criterion's, for instance, stay as they are), no loss scaler between, and no hook that could look at the
+        gradients in between."""
         opt = self.optimizer
         if self.scaler is not None or type(opt) not in (FusedAdamW, FusedSGD):
             return False
@@ -153,8 +154,8 @@ class Trainer:
         if opt._optimizer_step_pre_hooks or opt._optimizer_step_post_hooks or \
                 _torch_optimizer._global_optimizer_pre_hooks or _torch_optimizer._global_optimizer_post_hooks:
             return False
-        covered = {id(p) for group in opt.param_groups for p in group["params"]}
-        return all(id(p) in covered for p in self._params if p.grad is not None)
+        updated = {id(p) for group in opt.param_groups for p in group["params"] if p.grad is not None}
+        return updated == {id(p) for p in self._params if p.grad is not None}
 
     def _clip_factor(self):
         params = [p for p in self._params if p.grad is not None]

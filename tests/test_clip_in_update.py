@@ -54,3 +54,35 @@ def test_not_where_the_gradients_can_be_seen():
     patched = FusedAdamW(m.parameters())
     patched.step = lambda: None
     assert not _trainer(m, patched, clip=1.0)._folds_clipping()
+
+
+@pytest.mark.parametrize("make", [lambda p: FusedAdamW(p, lr=1e-2), lambda p: FusedSGD(p, lr=0.1)])
+def test_parameters_outside_the_model_are_not_clipped(make):
+    """An optimizer that also holds the criterion's parameter: clipping is that of the model's gradients alone."""
+
+    class Scaled(torch.nn.Module):
+
+        def __init__(self):
+            super().__init__()
+            self.scale = torch.nn.Parameter(torch.ones(1))
+
+        def forward(self, out, target):
+            return ((out * self.scale - target)**2).sum()
+
+    a, b = _model(), _model()
+    ca, cb = Scaled(), Scaled()
+    oa, ob = (make(list(m.parameters()) + list(c.parameters())) for m, c in ((a, ca), (b, cb)))
+    tr = Trainer(a, ca, oa, amp_dtype=None, clip=0.01, forward_fn=lambda m, x: (m(x["x"]), x["y"]))
+    for i in range(3):
+        g = torch.Generator().manual_seed(i)
+        batch = dict(x=torch.randn(8, 12, generator=g), y=torch.randn(8, 3, generator=g))
+        tr.step(batch)
+        cb(b(batch["x"]), batch["y"]).backward()
+        clip_grad_norm(list(b.parameters()), 0.01)
+        ob.step()
+        ob.zero_grad(set_to_none=True)
+        for p, q in zip([*a.parameters(), ca.scale], [*b.parameters(), cb.scale]):
+            assert torch.equal(p, q)
+    # without a gradient it is not in the way
+    (a(torch.randn(2, 12))).sum().backward()
+    assert tr._folds_clipping()
