@@ -813,9 +813,10 @@ std::vector<torch::Tensor> layer_norm_bwd_res(torch::Tensor dy, torch::Tensor x,
     check_rows(*dres);
     TORCH_CHECK(dres->sizes() == x.sizes() && dres->scalar_type() == x.scalar_type());
   }
-  if (x.size(1) > kWarpMaxBwd) return layer_norm_bwd_cta(dy, x, mean, rstd, gamma, has_res ? &*dres : nullptr);
   const int rows = x.size(0), H = x.size(1);
-  TORCH_CHECK(gamma.scalar_type() == torch::kFloat32 && gamma.is_contiguous() && gamma.numel() == H);
+  TORCH_CHECK(gamma.scalar_type() == torch::kFloat32 && gamma.is_contiguous() && gamma.numel() == H,
+              "norm parameters must be contiguous fp32 [H]");
+  if (H > kWarpMaxBwd) return layer_norm_bwd_cta(dy, x, mean, rstd, gamma, has_res ? &*dres : nullptr);
   gamma = aligned16(gamma);
   auto dx = torch::empty_like(x);
   auto f32 = x.options().dtype(torch::kFloat32);

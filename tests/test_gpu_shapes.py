@@ -63,6 +63,20 @@ def test_wide_layer_norm_with_residual(rows, H, dtype):
     assert ((y2.double() - ref).abs() <= UNIT[dtype] * ref.abs() + 1e-5).all()
 
 
+@pytest.mark.parametrize("H", [1280, 1288, 2048, 4096])           # both kernels of the backward
+def test_layer_norm_refuses_parameters_of_another_length(H):
+    ops, _ = _ops()
+    x, r = (torch.randn(4, H, device="cuda").bfloat16() for _ in range(2))
+    ones = torch.ones(H, device="cuda")
+    y, mean, rstd, total = ops.layer_norm_fwd(x, ones, ones, 1e-5, residual=r)
+    for bad in (ones[:H - 8], torch.ones(H + 8, device="cuda")):
+        for dres in (None, r):
+            with pytest.raises(RuntimeError, match="norm parameters"):
+                ops.layer_norm_bwd(y, total, mean, rstd, bad, dres=dres)
+        with pytest.raises(RuntimeError, match="norm parameters"):
+            ops.layer_norm_fwd(x, bad, ones, 1e-5)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("B,T,H,dh,causal,pad", [
     (1, 1, 1, 80, True, False),          # one row of one tile
