@@ -56,23 +56,25 @@ _SHADOWS = {}
 
 def shadow(param: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     """``param`` in ``dtype``; cached until the parameter changes (the fused optimizers refresh it
-    inside their update kernel, so in steady state no cast kernel runs)."""
+    inside their update kernel, so in steady state no cast kernel runs).  The copy outlives the call, so it is made with
+    inference mode off: an inference tensor could neither be saved for a backward pass nor be refreshed outside."""
     if param.dtype == dtype:
         return param.detach()
     key = (id(param), dtype)
     s = _SHADOWS.get(key)
     if s is not None and s.version == param._version and s.tensor.shape == param.shape and s.tensor.device == param.device:
         return s.tensor
-    base = param.detach()
-    if s is None or s.tensor.shape != base.shape or s.tensor.device != base.device:
-        s = _Shadow()
-        s.tensor = base.to(dtype)
-        s.version = param._version
-        _SHADOWS[key] = s
-        _register_shadow_finalizer(param, key)
-    elif s.version != param._version:
-        s.tensor.copy_(base)
-        s.version = param._version
+    with torch.inference_mode(False), torch.no_grad():
+        base = param.detach()
+        if s is None or s.tensor.shape != base.shape or s.tensor.device != base.device:
+            s = _Shadow()
+            s.tensor = base.to(dtype)
+            s.version = param._version
+            _SHADOWS[key] = s
+            _register_shadow_finalizer(param, key)
+        elif s.version != param._version:
+            s.tensor.copy_(base)
+            s.version = param._version
     return s.tensor
 
 
