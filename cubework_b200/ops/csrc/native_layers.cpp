@@ -59,7 +59,10 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
     g_native_launches += 1;
     auto r = gemm(x2, wa, false, out_in, bias, names[act], false, keep && act != 0);
     if (keep) {
-      ctx->save_for_backward({x2, w, wc, r[1].defined() ? r[1] : Tensor()});
+      // Saved as the Python function saves them.  The 16-bit copy of the weight is not the graph's (it is the parameter's, and
+      // stays): hooks on saved tensors, which may move them to the host, are not asked about it.
+      ctx->save_for_backward({x2, w, r[1].defined() ? r[1] : Tensor()});
+      ctx->saved_data["wc"] = wc;
       ctx->saved_data["out_in"] = out_in;
       ctx->saved_data["act"] = act;
       ctx->saved_data["b"] = bias.has_value() ? static_cast<int64_t>(bias->scalar_type()) : int64_t{-1};
@@ -73,7 +76,7 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor x2 = saved[0], w = saved[1], wc = saved[2], z = saved[3];
+    const Tensor x2 = saved[0], w = saved[1], z = saved[2], wc = ctx->saved_data["wc"].toTensor();
     const bool out_in = ctx->saved_data["out_in"].toBool();
     const int64_t act = ctx->saved_data["act"].toInt(), bt = ctx->saved_data["b"].toInt();
     const auto cd = wc.scalar_type();

@@ -94,3 +94,26 @@ def test_saved_tensor_hooks_see_what_is_kept():
     assert len(seen) >= 3
     y.float().sum().backward()
     assert x.grad is not None and w.grad is not None
+
+
+@pytest.mark.parametrize("params", [torch.float32, torch.bfloat16])
+def test_saved_tensor_hooks_see_the_same_tensors(params):
+    """What is offered to hooks (offloading) is what the Python functions offer, and not the weight's 16-bit copy besides."""
+    from cubework_b200 import ops
+    from cubework_b200.parallel.functional import _AddLayerNorm, _LocalLinear
+    x = torch.randn(24, 64, device="cuda").bfloat16().requires_grad_(True)
+    w, b = torch.randn(32, 64, device="cuda").to(params).requires_grad_(True), torch.zeros(32, device="cuda", dtype=params)
+    gamma = torch.ones(64, device="cuda", dtype=params)
+    qkv = torch.randn(2, 40, 3, 96, device="cuda").bfloat16().requires_grad_(True)
+
+    def offered(f):
+        seen = []
+        with torch.autocast("cuda", dtype=torch.bfloat16), \
+                torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append((tuple(t.shape), t.dtype)) or t, lambda t: t):
+            f()
+        return sorted((s, str(d)) for s, d in seen if 0 not in s)
+
+    assert offered(lambda: ops.native_linear(x, w, b, True, "relu")) == offered(lambda: _LocalLinear.apply(x, w, b, True, "relu", True))
+    assert offered(lambda: ops.native_linear(x, w, b, True, None)) == offered(lambda: _LocalLinear.apply(x, w, b, True, None, True))
+    assert offered(lambda: ops.native_norm(x, x, gamma, gamma, 1e-5)) == offered(lambda: _AddLayerNorm.apply(x, x, gamma, gamma, 1e-5))
+    assert offered(lambda: ops.attention_packed(qkv, True)) == offered(lambda: ops._AttentionFn.apply(qkv, True, None, 0.1))
