@@ -128,6 +128,15 @@ def mark_block_output(linear):
     inner.output_unused_in_recompute = True
 
 
+def add_norm(norm, x, contribution):
+    """``(x + contribution, norm(x + contribution))`` from one kernel, or from an add and the norm where the kernel would not
+    give the same: it adds in the compute dtype, so a stream that is held in more bits (fp32 under autocast) is added first."""
+    if x.dtype == contribution.dtype == ops.compute_dtype(x) and x.shape == contribution.shape:
+        return norm(x, residual=contribution)
+    x = x + contribution
+    return x, norm(x)
+
+
 def key_bias_from_mask(attention_mask, dtype=torch.float32):
     """``[B, T]`` mask of 1 (keep) / 0 (pad) -> additive bias over key positions, or None."""
     if attention_mask is None:

@@ -14,7 +14,7 @@ import torch.nn as nn
 from .. import module as cube_nn
 from .. import ops
 from ..parallel.loss import IGNORE_INDEX
-from .common import MLP, SelfAttention, key_bias_from_mask, mark_block_output, maybe_checkpoint, normal_init
+from .common import MLP, SelfAttention, add_norm, key_bias_from_mask, mark_block_output, maybe_checkpoint, normal_init
 
 
 def _init_kw(init_std):
@@ -99,9 +99,9 @@ class OPTDecoderLayer(nn.Module):
         if pending is None:
             n = self.self_attn_layer_norm(h)
         else:
-            h, n = self.self_attn_layer_norm(h, residual=pending)
+            h, n = add_norm(self.self_attn_layer_norm, h, pending)
         a, present = self._attend(n, key_bias, past_key_value, use_cache)
-        h, n = self.final_layer_norm(h, residual=self.dropout(a))
+        h, n = add_norm(self.final_layer_norm, h, self.dropout(a))
         out = self.ffn(n)
         return (h, out, present) if defer else (h + out, present)
 
@@ -181,7 +181,7 @@ class OPT(nn.Module):
             if use_cache:
                 cache += (present, )
         if pending is not None:
-            h = self.final_layer_norm(h, residual=pending)[1]
+            h = add_norm(self.final_layer_norm, h, pending)[1]
         elif defer:
             h = self.final_layer_norm(h)
         logits = self.lm_head(h)

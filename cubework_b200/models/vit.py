@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from .. import module as cube_nn
-from .common import MLP, SelfAttention, mark_block_output, maybe_checkpoint
+from .common import MLP, SelfAttention, add_norm, mark_block_output, maybe_checkpoint
 
 
 def _lin_kw():
@@ -68,8 +68,8 @@ class ViTBlock(nn.Module):
         if pending is None:
             n = self.norm1(x)
         else:
-            x, n = self.norm1(x, residual=pending)
-        x, n = self.norm2(x, residual=self.drop_path(self.attn(n)))
+            x, n = add_norm(self.norm1, x, pending)
+        x, n = add_norm(self.norm2, x, self.drop_path(self.attn(n)))
         out = self.drop_path(self.mlp(n))
         return (x, out) if defer else x + out
 
@@ -102,7 +102,7 @@ class VisionTransformer(nn.Module):
         pending = None
         for block in self.blocks:
             x, pending = block(x, pending, True)
-        return self.head(self.norm(x) if pending is None else self.norm(x, residual=pending)[1])
+        return self.head(self.norm(x) if pending is None else add_norm(self.norm, x, pending)[1])
 
 
 class MixupLoss(nn.Module):
