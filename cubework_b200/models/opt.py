@@ -14,7 +14,8 @@ import torch.nn as nn
 from .. import module as cube_nn
 from .. import ops
 from ..parallel.loss import IGNORE_INDEX
-from .common import MLP, SelfAttention, add_norm, key_bias_from_mask, mark_block_output, maybe_checkpoint, normal_init
+from .common import (MLP, SelfAttention, add_norm, is_plain, key_bias_from_mask, mark_block_output, maybe_checkpoint,
+                     normal_init)
 
 
 def _init_kw(init_std):
@@ -91,30 +92,33 @@ class OPTDecoderLayer(nn.Module):
             return self.self_attn.forward_cached(h, past_key_value, key_bias)
         return self.self_attn(h, key_bias), None
 
-    def _forward(self, h, key_bias=None, past_key_value=None, use_cache=False, pending=None, defer=False):
-        if not self.do_layer_norm_before:
-            a, present = self._attend(h, key_bias, past_key_value, use_cache)
-            h = self.self_attn_layer_norm(h + self.dropout(a))
-            return self.final_layer_norm(h + self.ffn(h)), present
+    def deferred(self, h, pending=None, key_bias=None, past_key_value=None, use_cache=False):
+        """``(stream, contribution, present)`` of a pre-LN layer: the layer without its last residual add, which is left to the
+        norm that follows (one kernel computes the sum and its normalised value).  ``pending`` is the contribution of the
+        layer before."""
         if pending is None:
             n = self.self_attn_layer_norm(h)
         else:
             h, n = add_norm(self.self_attn_layer_norm, h, pending)
         a, present = self._attend(n, key_bias, past_key_value, use_cache)
         h, n = add_norm(self.final_layer_norm, h, self.dropout(a))
-        out = self.ffn(n)
-        return (h, out, present) if defer else (h + out, present)
+        return h, self.ffn(n), present
 
-    def forward(self, h, key_bias=None, past_key_value=None, use_cache=False, pending=None, defer=False):
-        """``(h, present)``.  A pre-LN layer with ``defer`` leaves its last residual add to the norm that follows and
-        returns ``(stream, contribution, present)``; ``pending`` is such a contribution of the layer before (the norms
-        compute the sum and its normalised value in one kernel)."""
-        if self.gradient_checkpointing and self.training and not use_cache:
-            if defer:
-                out = maybe_checkpoint(lambda a, c, b: self._forward(a, b, pending=c, defer=True)[:2], True, h, pending, key_bias)
-                return (*out, None)
+    def _forward(self, h, key_bias=None, past_key_value=None, use_cache=False):
+        if self.do_layer_norm_before:
+            h, contribution, present = self.deferred(h, None, key_bias, past_key_value, use_cache)
+            return h + contribution, present
+        a, present = self._attend(h, key_bias, past_key_value, use_cache)
+        h = self.self_attn_layer_norm(h + self.dropout(a))
+        return self.final_layer_norm(h + self.ffn(h)), present
+
+    def recomputes(self, use_cache):
+        return self.gradient_checkpointing and self.training and not use_cache
+
+    def forward(self, h, key_bias=None, past_key_value=None, use_cache=False):
+        if self.recomputes(use_cache):
             return maybe_checkpoint(lambda a, b: self._forward(a, b)[0], True, h, key_bias), None
-        return self._forward(h, key_bias, past_key_value, use_cache, pending, defer)
+        return self._forward(h, key_bias, past_key_value, use_cache)
 
 
 class OPTLMLoss(nn.Module):
@@ -169,21 +173,26 @@ class OPT(nn.Module):
             key_bias = key_bias_from_mask(attention_mask)
         h = h + self.embed_positions(mask_full, past_len)
         cache = () if use_cache else None
-        defer, pending = self.final_layer_norm is not None, None
+        pending = None
         for idx, layer in enumerate(self.layers):
             if self.training and self.layerdrop > 0 and torch.rand(()).item() < self.layerdrop:
                 continue
             past = past_key_values[idx] if past_key_values is not None else None
-            if defer:
-                h, pending, present = layer(h, key_bias, past, use_cache, pending, True)
+            if is_plain(layer, OPTDecoderLayer) and layer.do_layer_norm_before:
+                if layer.recomputes(use_cache):
+                    h, pending = maybe_checkpoint(lambda a, c, b, f=layer.deferred: f(a, c, b)[:2], True, h, pending, key_bias)
+                    present = None
+                else:
+                    h, pending, present = layer.deferred(h, pending, key_bias, past, use_cache)
             else:
-                h, present = layer(h, key_bias, past, use_cache)
+                h, present = layer(h if pending is None else h + pending, key_bias, past, use_cache)
+                pending = None
             if use_cache:
                 cache += (present, )
-        if pending is not None:
-            h = add_norm(self.final_layer_norm, h, pending)[1]
-        elif defer:
-            h = self.final_layer_norm(h)
+        if self.final_layer_norm is None:
+            h = h if pending is None else h + pending
+        else:
+            h = self.final_layer_norm(h) if pending is None else add_norm(self.final_layer_norm, h, pending)[1]
         logits = self.lm_head(h)
         return (logits, cache) if use_cache else (logits, )
 

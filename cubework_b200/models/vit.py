@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from .. import module as cube_nn
-from .common import MLP, SelfAttention, add_norm, mark_block_output, maybe_checkpoint
+from .common import MLP, SelfAttention, add_norm, is_plain, mark_block_output, maybe_checkpoint
 
 
 def _lin_kw():
@@ -64,19 +64,22 @@ class ViTBlock(nn.Module):
                        inner_dropout=dropout)
         mark_block_output(self.mlp.dense_2)
 
-    def _forward(self, x, pending=None, defer=False):
+    def deferred(self, x, pending=None):
+        """``(stream, contribution)``: the block without its last residual add, which is left to the norm that follows (one
+        kernel computes the sum and its normalised value).  ``pending`` is the contribution of the block before."""
         if pending is None:
             n = self.norm1(x)
         else:
             x, n = add_norm(self.norm1, x, pending)
         x, n = add_norm(self.norm2, x, self.drop_path(self.attn(n)))
-        out = self.drop_path(self.mlp(n))
-        return (x, out) if defer else x + out
+        return x, self.drop_path(self.mlp(n))
 
-    def forward(self, x, pending=None, defer=False):
-        """The block's output; with ``defer`` its last residual add is left to the norm that follows and
-        ``(stream, contribution)`` is returned.  ``pending`` is such a contribution of the block before."""
-        return maybe_checkpoint(self._forward, self.checkpoint, x, pending, defer)
+    def _forward(self, x):
+        x, contribution = self.deferred(x)
+        return x + contribution
+
+    def forward(self, x):
+        return maybe_checkpoint(self._forward, self.checkpoint, x)
 
 
 class VisionTransformer(nn.Module):
@@ -101,7 +104,10 @@ class VisionTransformer(nn.Module):
         x = self.embed(pixel_values)
         pending = None
         for block in self.blocks:
-            x, pending = block(x, pending, True)
+            if is_plain(block, ViTBlock):
+                x, pending = maybe_checkpoint(block.deferred, block.checkpoint, x, pending)
+            else:
+                x, pending = block(x if pending is None else x + pending), None
         return self.head(self.norm(x) if pending is None else add_norm(self.norm, x, pending)[1])
 
 
