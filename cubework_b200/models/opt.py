@@ -178,12 +178,9 @@ class OPT(nn.Module):
             if self.training and self.layerdrop > 0 and torch.rand(()).item() < self.layerdrop:
                 continue
             past = past_key_values[idx] if past_key_values is not None else None
-            if is_plain(layer, OPTDecoderLayer) and layer.do_layer_norm_before:
-                if layer.recomputes(use_cache):
-                    h, pending = maybe_checkpoint(lambda a, c, b, f=layer.deferred: f(a, c, b)[:2], True, h, pending, key_bias)
-                    present = None
-                else:
-                    h, pending, present = layer.deferred(h, pending, key_bias, past, use_cache)
+            # (recomputation would keep both tensors of the pair)
+            if is_plain(layer, OPTDecoderLayer) and layer.do_layer_norm_before and not layer.recomputes(use_cache):
+                h, pending, present = layer.deferred(h, pending, key_bias, past, use_cache)
             else:
                 h, present = layer(h if pending is None else h + pending, key_bias, past, use_cache)
                 pending = None

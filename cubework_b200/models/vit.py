@@ -104,8 +104,8 @@ class VisionTransformer(nn.Module):
         x = self.embed(pixel_values)
         pending = None
         for block in self.blocks:
-            if is_plain(block, ViTBlock):
-                x, pending = maybe_checkpoint(block.deferred, block.checkpoint, x, pending)
+            if is_plain(block, ViTBlock) and not block.checkpoint:      # (recomputation would keep both tensors of the pair)
+                x, pending = block.deferred(x, pending)
             else:
                 x, pending = block(x if pending is None else x + pending), None
         return self.head(self.norm(x) if pending is None else add_norm(self.norm, x, pending)[1])

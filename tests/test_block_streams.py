@@ -147,3 +147,31 @@ def test_blocks_may_be_replaced(family):
             m.norm = torch.nn.LayerNorm(32, eps=1e-6)
             b[0].norm2 = torch.nn.LayerNorm(32, eps=1e-6)
             call(m, x)
+
+
+@pytest.mark.parametrize("family", list(FAMILIES))
+def test_recomputed_blocks_keep_one_tensor(family):
+    """With recomputation a block keeps its input for the backward pass and nothing else."""
+    make, inputs, blocks, call = FAMILIES[family]
+    kw = dict(checkpoint=True) if family == "vit" else dict(gradient_checkpointing=True)
+    m, ref, x = make(**kw).train(), make().train(), inputs()
+    ref.load_state_dict(m.state_dict())
+    from cubework_b200.models.common import _Recompute
+    kept, forward = [], _Recompute.forward
+
+    def counted(ctx, fn, *args):
+        kept.append(sum(torch.is_tensor(a) for a in args))
+        return forward(ctx, fn, *args)
+
+    _Recompute.forward = staticmethod(counted)
+    try:
+        out = call(m, x)
+    finally:
+        _Recompute.forward = staticmethod(forward)
+    assert kept == [1] * len(blocks(m))
+    out.square().sum().backward()
+    r = call(ref, x)
+    r.square().sum().backward()
+    assert torch.equal(out, r)
+    for (n, p), q in zip(m.named_parameters(), ref.parameters()):
+        assert torch.allclose(p.grad, q.grad, rtol=1e-4, atol=1e-6 * q.grad.abs().max().item()), n
