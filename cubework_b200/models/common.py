@@ -9,6 +9,7 @@ from torch.nn.modules.module import _has_any_global_hook
 from .. import module as cube_nn
 from .. import ops
 from ..parallel.facade import _PlainLayerNorm as PlainLayerNorm
+from ..parallel.functional import add_layer_norm
 from ..parallel.layers_1d import LayerNorm1D
 
 
@@ -135,18 +136,20 @@ def is_plain(module, *classes):
     """``module`` is one of ``classes`` with its own ``forward``, and nothing sees what it is called with: no hooks on it or on
     all modules, no trace being recorded.  Only then may a caller hand it other arguments than ``forward`` was documented
     with, or skip ``__call__``."""
-    return (type(module) in classes and "forward" not in module.__dict__ and not module._forward_hooks and
-            not module._forward_pre_hooks and not module._backward_hooks and not module._backward_pre_hooks and
-            not _has_any_global_hook() and torch._C._get_tracing_state() is None)
+    own = module.__dict__
+    return (module.__class__ in classes and "forward" not in own and not
+            (own["_forward_hooks"] or own["_forward_pre_hooks"] or own["_backward_hooks"] or own["_backward_pre_hooks"] or
+             _has_any_global_hook() or torch._C._get_tracing_state() is not None))
 
 
 def add_norm(norm, x, contribution):
     """``(x + contribution, norm(x + contribution))`` from one kernel, or from an add and the norm where the kernel would not
     give the same or be seen: it adds in the compute dtype, so a stream that is held in more bits (fp32 under autocast) is
     added first, and so is one whose norm is hooked or replaced."""
-    if x.dtype == contribution.dtype == ops.compute_dtype(x) and x.shape == contribution.shape and \
-            is_plain(norm, cube_nn.LayerNorm) and is_plain(norm.norm, PlainLayerNorm, LayerNorm1D):
-        return norm(x, residual=contribution)
+    if x.dtype == contribution.dtype == ops.compute_dtype(x) and x.shape == contribution.shape and is_plain(norm, cube_nn.LayerNorm):
+        inner = norm._modules["norm"]
+        if is_plain(inner, PlainLayerNorm, LayerNorm1D):     # (those of 2D and 3D parallelism add first as well)
+            return add_layer_norm(x, contribution, inner.weight, inner.bias, inner.eps)
     x = x + contribution
     return x, norm(x)
 
