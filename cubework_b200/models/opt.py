@@ -51,8 +51,8 @@ class OPTAttention(SelfAttention):
         b, t, w = qkv.shape
         heads = w // (3 * self.head_dim)
         packed = qkv.view(b, t, heads, 3 * self.head_dim)
-        if past_key_value is not None and ops.decode_ready(packed, *past_key_value, key_bias):
-            o, k, v = ops.decode_attention(packed, *past_key_value, key_bias)
+        if past_key_value is not None and ops.decode_ready(packed, past_key_value[0], past_key_value[1], key_bias):
+            o, k, v = ops.decode_attention(packed, past_key_value[0], past_key_value[1], key_bias)
             return self.dense(o), (k, v)
         q, k, v = packed.permute(0, 2, 1, 3).chunk(3, dim=-1)
         if past_key_value is None and ops.prefill_ready(packed, key_bias):

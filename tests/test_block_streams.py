@@ -175,3 +175,15 @@ def test_recomputed_blocks_keep_one_tensor(family):
     assert torch.equal(out, r)
     for (n, p), q in zip(m.named_parameters(), ref.parameters()):
         assert torch.allclose(p.grad, q.grad, rtol=1e-4, atol=1e-6 * q.grad.abs().max().item()), n
+
+
+def test_cached_attention_reads_the_first_two_entries():
+    """A cache entry may carry more than keys and values."""
+    env.load(mode=None)
+    torch.manual_seed(0)
+    m = opt.OPTAttention(32, 4)
+    x, t = torch.randn(2, 5, 32), torch.randn(2, 1, 32)
+    with torch.no_grad():
+        k, v = m.forward_cached(x)[1]
+        ref = m.forward_cached(t, (k, v))[0]
+        assert torch.equal(m.forward_cached(t, (k, v, "a note"))[0], ref)
