@@ -132,10 +132,26 @@ std::vector<torch::Tensor> gemm(torch::Tensor a, torch::Tensor b, bool trans_a, 
   return {out, z};
 }
 
+// The kernel that `gemm` takes for a product: the split-K factor on pairs of SMs (1 and above), 0 single CTAs, -1 the one that
+// streams the weights for a few rows.
+int gemm_pair_splits(const GemmArgs& g);         // gemm_pair_sm100.cu
+static int64_t gemm_route(int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b, bool out_f32, bool want_z, bool split) {
+  if (!trans_a && trans_b && !out_f32 && M <= kSkinnyRows) return -1;
+  GemmArgs g;
+  char z = 0;
+  g.z_out = want_z ? &z : nullptr;
+  g.M = static_cast<int>(M); g.N = static_cast<int>(N); g.K = static_cast<int>(K);
+  g.out_f32 = out_f32;
+  g.allow_split_k = split;
+  g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  return gemm_pair_splits(g);
+}
+
 }  // namespace cw
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &cw::gemm);
+  m.def("gemm_route", &cw::gemm_route);
   m.def("status_device_ptr", &cw::status_device_ptr);
   m.def("read_status", &cw::read_status);
   m.def("layer_norm_fwd", &cw::layer_norm_fwd);
