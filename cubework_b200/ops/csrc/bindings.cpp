@@ -108,8 +108,12 @@ std::vector<torch::Tensor> gemm(torch::Tensor a, torch::Tensor b, bool trans_a, 
   if (K == 0) { out.zero_(); return {out, z}; }
   torch::Tensor bias_f;
   GemmArgs g;
-  const bool skinny = !trans_a && trans_b && !out_f32 && M <= kSkinnyRows;      // the rule of gemm_launch
-  if (skinny && bias.has_value() && bias->defined() && bias->scalar_type() == a.scalar_type() && bias->is_contiguous()) {
+  g.M = static_cast<int>(M); g.N = static_cast<int>(N); g.K = static_cast<int>(K);
+  g.trans_a = trans_a; g.trans_b = trans_b;
+  g.is_bf16 = a.scalar_type() == torch::kBFloat16;
+  g.out_f32 = out_f32;
+  g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  if (gemm_is_skinny(g) && bias.has_value() && bias->defined() && bias->scalar_type() == a.scalar_type() && bias->is_contiguous()) {
     TORCH_CHECK(bias->numel() == N && bias->is_cuda(), "bias must have one value per output column");
     g.bias16 = bias->data_ptr();
   } else if (bias.has_value() && bias->defined()) {
@@ -120,13 +124,8 @@ std::vector<torch::Tensor> gemm(torch::Tensor a, torch::Tensor b, bool trans_a, 
   g.a = a.data_ptr(); g.b = b.data_ptr(); g.out = out.data_ptr();
   g.z_out = want_z ? z.data_ptr() : nullptr;
   g.bias = bias_f.defined() ? bias_f.data_ptr<float>() : nullptr;
-  g.M = static_cast<int>(M); g.N = static_cast<int>(N); g.K = static_cast<int>(K);
-  g.trans_a = trans_a; g.trans_b = trans_b;
-  g.is_bf16 = a.scalar_type() == torch::kBFloat16;
-  g.out_f32 = out_f32;
   g.act = act_code(act);
   g.allow_split_k = g.act == kActNone && !want_z;
-  g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   g.status = g_status_dev;
   gemm_launch(g, at::cuda::getCurrentCUDAStream());
   return {out, z};
@@ -136,15 +135,15 @@ std::vector<torch::Tensor> gemm(torch::Tensor a, torch::Tensor b, bool trans_a, 
 // streams the weights for a few rows.
 int gemm_pair_splits(const GemmArgs& g);         // gemm_pair_sm100.cu
 static int64_t gemm_route(int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b, bool out_f32, bool want_z, bool split) {
-  if (!trans_a && trans_b && !out_f32 && M <= kSkinnyRows) return -1;
   GemmArgs g;
   char z = 0;
   g.z_out = want_z ? &z : nullptr;
   g.M = static_cast<int>(M); g.N = static_cast<int>(N); g.K = static_cast<int>(K);
+  g.trans_a = trans_a; g.trans_b = trans_b;
   g.out_f32 = out_f32;
   g.allow_split_k = split;
   g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  return gemm_pair_splits(g);
+  return gemm_is_skinny(g) ? -1 : gemm_pair_splits(g);
 }
 
 }  // namespace cw

@@ -369,12 +369,20 @@ static void launch_skinny(const GemmArgs& g, cudaStream_t stream) {
   const T* b16 = reinterpret_cast<const T*>(g.bias16);
   T* y = reinterpret_cast<T*>(g.out);
   T* z = reinterpret_cast<T*>(g.z_out);
-  // 16 warps share a long K: with eight, each made four dependent rounds of loads at K = 8192 (2048 x 8192 weights: 9.7 us)
+  // 16 warps share K instead of eight where that does not cost a wave, two CTAs of eight or one of 16 per SM (microseconds with
+  // eight and 16): up to one CTA per SM (2304 x 9216, 8 rows 12.9 and 10.6, 16 rows 21.8 and 14.8; 2400 columns 13.3 and 15.8, 22.0
+  // and 26.0) and, for few rows and a long K, three (5120 x 8192, 8 rows: 23.8 and 21.9, x 20480: 52.8 and 47.1; 7168: 57.7 and 63.1;
+  // 6144 x 2048: 8.5 and 9.2).  With more than 16 rows a warp has one step in flight: up to two CTAs per SM (4736 x 2048, 32
+  // rows: 12.4 and 9.2; 8192 x 2048 14.9 and 16.1) and always for a long K (12288 x 8192: 86 and 63).
+  const int sms = g.num_sms;
+  const bool wide = g.M <= 8    ? grid <= sms || (g.K >= 8192 && grid > 2 * sms && grid <= 3 * sms)
+                    : g.M <= 16 ? grid <= sms
+                                : grid <= 2 * sms || g.K >= 8192;
 #define LAUNCH_SKINNY(NT, W) \
   skinny_gemm_kernel<T, NT, W><<<grid, 32 * W, 0, stream>>>(x, w, g.bias, b16, y, z, g.M, g.N, g.K, g.act)
-  if (g.M <= 8) { if (g.K >= 4096) LAUNCH_SKINNY(1, 16); else LAUNCH_SKINNY(1, 8); }
-  else if (g.M <= 16) { if (g.K >= 4096) LAUNCH_SKINNY(2, 16); else LAUNCH_SKINNY(2, 8); }
-  else { if (g.K >= 4096) LAUNCH_SKINNY(4, 16); else LAUNCH_SKINNY(4, 8); }
+  if (g.M <= 8) { if (wide) LAUNCH_SKINNY(1, 16); else LAUNCH_SKINNY(1, 8); }
+  else if (g.M <= 16) { if (wide) LAUNCH_SKINNY(2, 16); else LAUNCH_SKINNY(2, 8); }
+  else { if (wide) LAUNCH_SKINNY(4, 16); else LAUNCH_SKINNY(4, 8); }
 #undef LAUNCH_SKINNY
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }

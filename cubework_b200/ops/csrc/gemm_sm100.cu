@@ -392,7 +392,7 @@ static void dispatch_major(bool ak, bool bk, const CUtensorMap& ta, const CUtens
 // Host entry.  a: [M,K] (trans_a=false) or [K,M]; b: [K,N] (trans_b=false) or [N,K]; both contiguous 2-D.
 void gemm_launch(const GemmArgs& g, cudaStream_t stream) {
   // a handful of rows against row-major weights: the weight-streaming kernel of decode_sm100.cu
-  if (!g.trans_a && g.trans_b && !g.out_f32 && g.M <= kSkinnyRows) {
+  if (gemm_is_skinny(g)) {
     skinny_gemm_launch(g, stream);
     return;
   }

@@ -81,6 +81,10 @@ def test_decode_ready_refuses():
 @pytest.mark.parametrize("M,N,K,act", [
     (1, 1, 8, None), (1, 768, 768, "relu"), (8, 2048, 2048, None), (9, 2304, 768, "gelu"), (16, 50, 4104, None),
     (17, 2048, 8192, "relu"), (32, 1000, 520, "gelu"), (33, 1000, 520, "gelu"), (3, 250, 1001, None),
+    (16, 2368, 264, None), (16, 2376, 264, "relu"), (32, 4736, 264, "gelu"), (32, 4744, 264, None),      # ends of the rule for the warps
+    (17, 9472, 136, None), (17, 9480, 136, "relu"),                                                       # ... and for the kernel
+    (9, 16392, 2048, None), (9, 16392, 2056, "gelu"), (8, 20488, 1024, None), (8, 20488, 1016, "relu"),
+    (9, 16392, 1024, None), (8, 4744, 8192, "relu"), (5, 7112, 8192, None), (32, 4744, 8192, "gelu"),
 ])
 def test_skinny_gemm(dtype, M, N, K, act):
     ops = _ops()
@@ -88,6 +92,10 @@ def test_skinny_gemm(dtype, M, N, K, act):
     x = torch.randn(M, K, generator=g, device="cuda").to(dtype)
     w = (torch.randn(N, K, generator=g, device="cuda") / math.sqrt(K)).to(dtype)
     b = torch.randn(N, generator=g, device="cuda")
+    streams = M <= 32 and (M <= 16 or N <= 9472) and (M <= 8 or M > 16 or N <= 16384 or 1024 < K <= 2048) and \
+        (M > 8 or N <= 20480 or 1024 <= K <= 8192)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert (ops.ext.require().gemm_route(M, N, K, False, True, False, True, False) == -1) == streams
     y, z = ops.gemm(x, w, trans_b=True, bias=b, act=act, pre_act_out=True)
     ref = x.double() @ w.double().t() + b.double()
     # one rounding of the result, and fp32 sums of K products of unit variance / K
