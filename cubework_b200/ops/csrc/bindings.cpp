@@ -134,14 +134,16 @@ std::vector<torch::Tensor> gemm(torch::Tensor a, torch::Tensor b, bool trans_a, 
 // The kernel that `gemm` takes for a product: the split-K factor on pairs of SMs (1 and above), 0 single CTAs, -1 the one that
 // streams the weights for a few rows.
 int gemm_pair_splits(const GemmArgs& g);         // gemm_pair_sm100.cu
-static int64_t gemm_route(int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b, bool out_f32, bool want_z, bool split) {
+static int64_t gemm_route(int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b, const std::string& act, bool out_f32,
+                          bool want_z) {
   GemmArgs g;
   char z = 0;
   g.z_out = want_z ? &z : nullptr;
   g.M = static_cast<int>(M); g.N = static_cast<int>(N); g.K = static_cast<int>(K);
   g.trans_a = trans_a; g.trans_b = trans_b;
   g.out_f32 = out_f32;
-  g.allow_split_k = split;
+  g.act = act_code(act);
+  g.allow_split_k = g.act == kActNone && !want_z;
   g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   return gemm_is_skinny(g) ? -1 : gemm_pair_splits(g);
 }

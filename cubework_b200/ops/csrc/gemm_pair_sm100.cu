@@ -394,20 +394,39 @@ static void dispatch_pair(bool ak, bool bk, const CUtensorMap& ta, const CUtenso
   else launch_pair<false, false, InT, OUT_F32>(ta, tb, to, tz, p, pairs, s);
 }
 
-// Split-K factor for pairs, or 0 where the single-CTA kernel stays: products with an extent that half a tile covers, and
-// those of so few k-blocks that the pair's start-up (the cluster barriers) is not paid for (999 x 768 x 768, 12 k-blocks in
-// one wave: 15.4 us single, 17.4 in pairs; 2000 x 2048 x 2048, 32 k-blocks: 23.6 both; 6304 x 3072 x 768, 5 waves of 12:
-// 35.8 and 33.8).
+// k-blocks from which a 16-bit product is faster in pairs, by its waves over 74 pairs.  Pairs win 7 to 10 % of the MMAs' time and
+// lose 1.6 us at the start (cluster barriers) and some of a short tile's epilogue, most with GELU.  Time in pairs over time in single
+// CTAs, 2172 shapes in turn; K-major B (forward) / MN-major B (data gradient):
+//   one wave    32 k-blocks 1.09 / 1.06, 48 1.07 / 1.04, 80 1.02 / 1.00, 128 1.00 / 0.98
+//   two waves   16 k-blocks 1.04 / 0.99, 25 1.03 / 1.00, 40 0.99 / 0.97, 80 0.92 / 0.93
+//   three       12 k-blocks 1.01 / 0.97, 20 1.01 / 0.98, 25 0.99 / 0.97; with a pre-activation copy 0.97 from 12 on
+//   more        8 k-blocks 1.06 / 0.99, 12 0.96 / 0.93, 16 0.94 / 0.92; with GELU 12 1.07, 16 1.02, 20 0.97, 25 0.97
+static int pair_min_kb(const GemmArgs& g, int64_t waves) {
+  const bool kmajor = g.trans_b;
+  const int kb = waves == 1 ? (kmajor ? 128 : 72) : waves == 2 ? (kmajor ? 40 : 24) : waves == 3 && kmajor && g.z_out == nullptr ? 24 : 12;
+  return g.act == kActGelu ? std::max(kb, 20) : kb;
+}
+
+// Split-K factor for pairs, or 0 where the single-CTA kernel stays: products with an extent that half a tile covers, those
+// of too few k-blocks, and those that take more waves of pairs than of single CTAs (333 x 10240 x 2560: two waves instead of one,
+// 33.9 us and 20.3).
 // A weight gradient has few, very long tiles (K = tokens), so K is split to fill the waves: a wave costs the k-blocks of a
 // tile plus about 3 for what does not overlap, a split about 2 k-blocks per million outputs for its partial sums.  Best of
-// a sweep: 6400 x 1600 x 32768 two splits, 1600 x 1600 three, 768 x 768 x 50432 eight, 4800 x 1600 x 32768 one.
+// a sweep: 6400 x 1600 x 32768 two splits, 1600 x 1600 three, 768 x 768 x 50432 eight, 4800 x 1600 x 32768 one.  With fp32
+// outputs pairs pay from 32 k-blocks over all waves (2048 x 2048 x 2000: 18.4 and 17.9 us), of at least 8 each (50304 x 768, 6
+// k-blocks: 42.9 and 47.4; 8: 51.6 and 50.7); with split K from 28 (768 x 768 x 2000, 4 splits of 8: 10.9 and 12.0; 2304 x 768 x
+// 3000, 2 of 24: 17.9 and 18.1; x 4096, 2 of 32: 21.1 and 20.8).
 int gemm_pair_splits(const GemmArgs& g) {
   if (g.M <= kBM || g.N <= kPairBN / 2 || (g.out_f32 && g.z_out != nullptr)) return 0;
   const int kb = (g.K + kBK - 1) / kBK, pairs = g.num_sms / 2;
   const int64_t tiles = static_cast<int64_t>((g.M + 2 * kBM - 1) / (2 * kBM)) * ((g.N + kPairBN - 1) / kPairBN);
-  if ((tiles + pairs - 1) / pairs * kb < 32) return 0;
-  const int max_split = (g.out_f32 && g.allow_split_k) ? std::min(32, std::max(1, kb / 8)) : 1;
-  int best = 1;
+  const int64_t waves1 = (tiles + pairs - 1) / pairs;
+  const int64_t single = (static_cast<int64_t>((g.M + kBM - 1) / kBM) * ((g.N + kPairBN - 1) / kPairBN) + g.num_sms - 1) / g.num_sms;
+  const bool more_waves = waves1 * 14 > single * 15;
+  if (!g.out_f32) return more_waves || kb < pair_min_kb(g, waves1) ? 0 : 1;
+  const int max_split = g.allow_split_k ? std::min(32, std::max(1, kb / 8)) : 1;
+  int best = 1, best_per = kb;
+  int64_t best_waves = waves1;
   double best_time = 0.0;
   for (int sp = 1; sp <= max_split; ++sp) {
     const int per = (kb + sp - 1) / sp;
@@ -415,9 +434,10 @@ int gemm_pair_splits(const GemmArgs& g) {
     const int64_t waves = (tiles * sp + pairs - 1) / pairs;
     double t = static_cast<double>(waves) * (per + 3.0);
     if (sp > 1) t += 2e-6 * sp * g.M * static_cast<double>(g.N) + 4.0;       // 4: the memset
-    if (sp == 1 || t < best_time) { best = sp; best_time = t; }
+    if (sp == 1 || t < best_time) { best = sp; best_time = t; best_per = per; best_waves = waves; }
   }
-  return best;
+  if (best > 1) return best_waves * best_per >= 28 ? best : 0;
+  return more_waves || kb < 8 || waves1 * kb < 32 ? 0 : 1;
 }
 
 void gemm_pair_launch(const GemmArgs& g, int splits, cudaStream_t stream) {

@@ -95,7 +95,7 @@ def test_skinny_gemm(dtype, M, N, K, act):
     streams = M <= 32 and (M <= 16 or N <= 9472) and (M <= 8 or M > 16 or N <= 16384 or 1024 < K <= 2048) and \
         (M > 8 or N <= 20480 or 1024 <= K <= 8192)
     if torch.cuda.get_device_properties(0).multi_processor_count == 148:
-        assert (ops.ext.require().gemm_route(M, N, K, False, True, False, True, False) == -1) == streams
+        assert (ops.ext.require().gemm_route(M, N, K, False, True, act or "", False, True) == -1) == streams
     y, z = ops.gemm(x, w, trans_b=True, bias=b, act=act, pre_act_out=True)
     ref = x.double() @ w.double().t() + b.double()
     # one rounding of the result, and fp32 sums of K products of unit variance / K

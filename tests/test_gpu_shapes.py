@@ -120,27 +120,31 @@ def test_attention_tiles(dtype, B, T, H, dh, causal, pad):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("trans_a,trans_b", [(False, True), (False, False), (True, False), (True, True)])
-@pytest.mark.parametrize("M,N,K,pairs", [
-    (256, 256, 64, False),         # one tile, one k-block
-    (264, 64, 72, False),
-    (1000, 1608, 200, False),
-    (33, 50304, 136, False),
-    (256, 256, 2048, True),        # one tile, the fewest k-blocks that the rule sends to pairs
-    (264, 136, 2056, True),        # a second row block of 8 rows, the narrowest tile, a ragged last k-block
-    (1000, 1608, 2088, True),      # ragged in every extent
-    (4096, 1600, 1600, True),      # two waves, a last tile of 64 columns
-    (2048, 776, 4104, True),       # more k-blocks than stages
-    (136, 50304, 776, True),       # almost half of every row block empty, several tiles per pair
+@pytest.mark.parametrize("M,N,K,pairs,pairs32", [       # whether 16-bit and fp32 outputs go to the kernel on pairs
+    (256, 256, 64, False, False),         # one tile, one k-block
+    (264, 64, 72, False, False),
+    (1000, 1608, 200, False, False),
+    (33, 50304, 136, False, False),
+    (333, 10240, 2056, False, False),     # one wave of single CTAs, two of pairs
+    (256, 256, 8128, False, False),       # one k-block less than the rule asks for
+    (256, 256, 8192, True, False),        # one tile
+    (264, 136, 8200, True, False),        # a second row block of 8 rows, the narrowest tile, a ragged last k-block
+    (1000, 1608, 8200, True, True),       # ragged in every extent; split K
+    (4096, 1600, 2600, True, True),       # two waves, a last tile of 64 columns
+    (2048, 776, 8200, True, True),        # one wave of long tiles
+    (136, 50304, 1544, True, True),       # almost half of every row block empty, several tiles per pair
+    (4096, 8192, 776, True, True),        # short tiles in many waves
 ])
-def test_gemm_on_pairs(dtype, trans_a, trans_b, M, N, K, pairs):
+def test_gemm_on_pairs(dtype, trans_a, trans_b, M, N, K, pairs, pairs32):
     ops, ext = _ops()
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     pad = lambda n: (n + 7) // 8 * 8
     M = pad(M) if trans_a else M
     a = torch.randn((K, M) if trans_a else (M, K), generator=g, device="cuda").to(dtype)
     b = torch.randn((N, K) if trans_b else (K, N), generator=g, device="cuda").to(dtype)
-    for f32 in (False, True):
-        assert (ext.require().gemm_route(M, N, K, trans_a, trans_b, f32, False, True) > 0) == pairs
+    route = ext.require().gemm_route
+    assert (route(M, N, K, trans_a, True, "", False, False) > 0) == pairs and (route(M, N, K, trans_a, trans_b, "", True, False) > 0) == pairs32
+    assert not pairs or route(M, N, K, trans_a, trans_b, "", False, False) > 0
     ref = (a.float().t() if trans_a else a.float()) @ (b.float().t() if trans_b else b.float())
     out32 = ops.gemm(a, b, trans_a, trans_b, out_dtype=torch.float32)
     out = ops.gemm(a, b, trans_a, trans_b)
@@ -153,19 +157,20 @@ def test_gemm_on_pairs(dtype, trans_a, trans_b, M, N, K, pairs):
 @pytest.mark.parametrize("act", [None, "gelu", "relu"])
 @pytest.mark.parametrize("M,N,K", [
     (300, 1600, 264), (520, 1000, 264), (4096, 160, 264), (700, 2300, 264), (260, 60, 264),      # the single-CTA kernel
-    (300, 1600, 2056),             # one live chunk of 64 columns in the last tile, rows for only half of a cluster
-    (520, 1000, 2056),             # a half chunk at the matrix's end
-    (4096, 160, 2056),             # one tile wide, three chunks of which the last is half
-    (700, 2300, 2056),             # a row pitch that TMA cannot store
-    (260, 132, 2056),              # ... with one row quarter of four rows and a chunk of four columns
-    (256, 260, 2056),              # ... with a last tile of four columns
-    (6304, 1544, 776),             # several tiles per pair: both accumulators and their hand-over
+    (300, 1600, 8200),             # one live chunk of 64 columns in the last tile, rows for only half of a cluster
+    (520, 1000, 8200),             # a half chunk at the matrix's end
+    (4096, 160, 8200),             # one tile wide, three chunks of which the last is half
+    (700, 2300, 8200),             # a row pitch that TMA cannot store
+    (260, 132, 8200),              # ... with one row quarter of four rows and a chunk of four columns
+    (256, 260, 8200),              # ... with a last tile of four columns
+    (6304, 1544, 1544),            # several tiles per pair: both accumulators and their hand-over
 ])
 def test_gemm_on_pairs_epilogue(M, N, K, act, dtype):
     """Bias, activation and the pre-activation copy: whole chunks, half chunks at a tile's or the matrix's end, and a row
     pitch that TMA cannot store, in the kernel for pairs of SMs and in the one for single CTAs."""
     ops, ext = _ops()
-    assert (ext.require().gemm_route(M, N, K, False, True, False, True, False) > 0) == (K != 264)
+    route = ext.require().gemm_route
+    assert all((route(M, N, K, False, True, act or "", False, z) > 0) == (K != 264) for z in (False, True))
     g = torch.Generator(device="cuda").manual_seed(M + N)
     a = torch.randn(M, K, generator=g, device="cuda").to(dtype)
     b = (torch.randn(N, K, generator=g, device="cuda") / math.sqrt(K)).to(dtype)
@@ -176,8 +181,8 @@ def test_gemm_on_pairs_epilogue(M, N, K, act, dtype):
     y1 = ext.gemm(a, b, False, True, bias, act, dtype, False)
     y32 = ext.gemm(a, b, False, True, bias, act, torch.float32, False)
     ext.check_status()
-    # K / 16 accumulations, each rounding a running sum below 8 to 24 bits: 130 * 2^-24 * 8 at K = 2056
-    u = UNIT[dtype]
-    assert ((z.double() - z_ref).abs() <= u * z_ref.abs() + 1e-4).all()
-    assert ((y.double() - y_ref).abs() <= u * y_ref.abs() + 1e-4).all() and torch.equal(y, y1)
-    assert ((y32.double() - y_ref).abs() <= 1e-4).all()
+    # K / 16 accumulations, each rounding a running sum below 8 to 24 bits, and the activation's error
+    u, acc = UNIT[dtype], K / 16 * 2.0**-24 * 8 + 1e-5
+    assert ((z.double() - z_ref).abs() <= u * z_ref.abs() + acc).all()
+    assert ((y.double() - y_ref).abs() <= u * y_ref.abs() + acc).all() and torch.equal(y, y1)
+    assert ((y32.double() - y_ref).abs() <= acc).all()
