@@ -305,6 +305,10 @@ __global__ void __launch_bounds__(kNT, VPT == 1 ? 4 : VPT <= 3 ? 2 : 1) ln_bwd_k
 // (reference: `x = x + dropout(...)` followed by `norm(x)`, benchmark/gpt2/gpt2.py:179-186): forward writes the sum
 // and its normalised value, backward adds the gradient that reaches the sum directly.
 constexpr int kWarpRows = 8;                 // warps (rows in flight) per CTA
+// The backward of rows above 1280 columns takes a CTA per row, four per SM, with the parameter gradients in registers: by
+// warps, sixteen rows per SM wait for their loads (32768 x 1600 with a residual 163 us, 120 by CTAs; 4096 x 2048 56 and 32;
+// at 1280 65 and 60, without a residual 52 and 54; at 768 99 and 136).
+constexpr int kWarpMaxBwd = 1280;
 
 template <typename T, int NV, bool HAS_RES, typename P>
 __global__ void __launch_bounds__(32 * kWarpRows)
@@ -389,10 +393,10 @@ ln_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res, const P* 
   }
 }
 
-// Backward of the above.  Each warp keeps the dgamma / dbeta partial sums of its rows in a shared-memory strip of its
-// own (in registers they cost 112 registers per thread at H = 1600 and held the kernel at eight warps per SM, where it
-// was bound by latency); the warps of a CTA are added up at the end and the CTA writes one partial row (summed by
-// colsum_kernel).
+// Backward of the above, for rows of up to kWarpMaxBwd columns.  Each warp keeps the dgamma / dbeta partial sums of its rows
+// in a shared-memory strip of its own (in registers they would take 2 * H / 32 per thread, 80 at H = 1280, and hold the kernel
+// at eight warps per SM, where it is bound by latency); the warps of a CTA are added up at the end and the CTA writes one
+// partial row (summed by colsum_kernel).
 template <typename T, int NV, bool HAS_RES>
 __global__ void __launch_bounds__(32 * kWarpRows, 2)
 ln_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ mean,
@@ -511,7 +515,7 @@ static void launch_ln_bwd_warp(int grid, size_t smem, cudaStream_t stream, const
   auto kern = ln_bwd_warp_kernel<T, NV, HAS_RES>;
   static bool done = false;
   if (!done) {
-    C10_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarpRows * 2 * 2048 * 4));
+    C10_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarpRows * 2 * kWarpMaxBwd * 4));
     done = true;
   }
   kern<<<grid, 32 * kWarpRows, smem, stream>>>(reinterpret_cast<const T*>(dy), reinterpret_cast<const T*>(x), mean, rstd, gamma,
@@ -733,10 +737,6 @@ constexpr int kWarpMaxH = 2048;
     DISPATCH_NV((x).size(1), __VA_ARGS__)                          \
   }
 
-// The backward of rows above 1280 columns takes a CTA per row, four per SM, with the parameter gradients in registers: by
-// warps, sixteen rows per SM wait for their loads (32768 x 1600 with a residual 163 us, 120 by CTAs; 4096 x 2048 56 and 32;
-// at 1280 65 and 60, without a residual 52 and 54; at 768 99 and 136).
-constexpr int kWarpMaxBwd = 1280;
 #define DISPATCH_16_NV_BWD(x, ...)                                 \
   {                                                                \
     const int need_ = ((x).size(1) / 8 + 31) / 32;                 \
