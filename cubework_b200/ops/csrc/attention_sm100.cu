@@ -168,11 +168,11 @@ __device__ __forceinline__ bool mbar_wait_ol(uint64_t* bar, uint32_t parity, vol
 }
 // ---------------------------------------------------------------------------------------------------------
 // Forward: persistent CTAs of eleven warps that take two neighbouring query tiles ("lanes" w = 0, 1) of one (batch, head)
-// and share their K / V blocks.
+// and share their K / V blocks, or the odd last tiles of two heads (FwdItem).
 //   softmax group   warps 4w .. 4w+3: thread r owns query row r; two passes over the scores in TMEM (maximum, then
 //                   exponentials); P goes back to TMEM as 16 bits and is the A operand of P V from there
 //   MMA issuers     warps 8, 9: S_w = Q_w K_j^T and O_w += P_w V_j
-//   TMA producer    warp 10: Q_w, one ring of four stages that K and V blocks share, key bias (ring of four)
+//   TMA producer    warp 10: Q_w, one ring of four stages that K and V blocks share, key bias (ring of eight)
 // What bounds it: 128 x 128 scores take 1024 clocks of the exponential units, and at a head dim of 128 the two products as
 // many of the tensor cores.  Two lanes keep both busy: while one group waits for a product the other computes.
 //   head dim <= 64  P has TMEM columns of its own, so the next scores are computed while the group still works on the last
@@ -186,7 +186,7 @@ __device__ __forceinline__ bool mbar_wait_ol(uint64_t* bar, uint32_t parity, vol
 // then P is relative to the older maximum, which is exact up to the same relative rounding, and stays below 256.
 // TMEM: S_w at 128 w; head dim <= 64: O_w at 256 + 64 w, P_w at 384 + 64 w; above: P_w at 128 w, O_w at 256 + 128 w.
 constexpr int kFwdThreads = 352;
-constexpr int kFwdRing = 4, kFwdBiasRing = 4;
+constexpr int kFwdRing = 4, kFwdBiasRing = 8;
 constexpr float kRescaleLog2 = 8.f;
 template <int DP>
 constexpr int fwd_stage_bytes() { return DP <= 64 ? 8 * 32 * DP * 2 : 0; }     // output rows that are no multiple of 16 bytes
@@ -194,6 +194,46 @@ template <int DP>
 constexpr int fwd_smem() {
   return (2 + kFwdRing) * ((DP + 63) / 64) * kBlk * 128 + fwd_stage_bytes<DP>() + kFwdBiasRing * kBlk * 4 + 512 + 1024;
 }
+// A work item: two tiles, lane w's being query block qb[w] of (batch, head) bh[w] with n[w] key blocks (0: the lane has none).
+// Neighbouring tiles of one head share their K / V blocks; lane 0 never has more of them than lane 1 unless lane 1 has none.  The
+// last tile of an odd number has no neighbour.  With PAIR_ODD it goes with that of the next head (`solo`): each lane then has K / V
+// blocks of its own, which come in turn.
+__host__ __device__ inline int fwd_odd_items(int n_qb, int bh_total, bool pair_odd) {
+  return (n_qb & 1) * (pair_odd ? (bh_total + 1) / 2 : bh_total);
+}
+__host__ __device__ inline int fwd_items(int n_qb, int bh_total, bool pair_odd) {
+  return fwd_odd_items(n_qb, bh_total, pair_odd) + n_qb / 2 * bh_total;
+}
+template <bool PAIR_ODD>
+struct FwdItem {
+  int qb[2], bh[2], n[2];
+  int blocks;                      // K / V blocks that go through the ring
+  bool solo;
+  __device__ FwdItem(int t, int n_qb, int bh_total, int causal) {
+    if constexpr (PAIR_ODD) {
+      const int n_odd = fwd_odd_items(n_qb, bh_total, true);
+      if (t < n_odd) {
+        qb[0] = qb[1] = n_qb - 1;
+        bh[0] = 2 * t;
+        bh[1] = bh[0] + 1;
+        solo = bh[1] < bh_total;
+        n[0] = n_qb;
+        n[1] = solo ? n_qb : 0;
+        blocks = n[0] + n[1];
+        return;
+      }
+      t += (n_qb & 1) * bh_total - n_odd;
+    }
+    const int pair = t / bh_total;
+    bh[0] = bh[1] = t - pair * bh_total;
+    qb[0] = 2 * ((n_qb + 1) / 2 - 1 - pair);
+    qb[1] = qb[0] + 1;
+    solo = false;
+    n[0] = causal ? qb[0] + 1 : n_qb;
+    n[1] = qb[1] >= n_qb ? 0 : (causal ? qb[1] + 1 : n_qb);
+    blocks = n[1] > n[0] ? n[1] : n[0];
+  }
+};
 struct FwdBars {
   uint64_t q_full[2], q_empty[2];
   uint64_t kv_full[kFwdRing], kv_empty[kFwdRing];
@@ -201,7 +241,7 @@ struct FwdBars {
   int bias_nz[kFwdBiasRing];       // the key bias of this ring slot has a non-zero entry
 };
 
-template <typename T, int DP>
+template <typename T, int DP, bool PAIR_ODD>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, AttnParams p) {
@@ -240,12 +280,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   const uint32_t tmem = *tmem_slot;
 
   const int n_qb = (p.T + kBlk - 1) / kBlk;
-  const int n_pair = (n_qb + 1) / 2;
   const int bh_total = p.B * p.H;
-  const int items = n_pair * bh_total;
-  // key blocks of a tile; 0 when the pair has no such tile.  Lane 0 never has more than lane 1 unless lane 1 has none.
-  auto n_kv_of = [&](int qb) { return qb >= n_qb ? 0 : (p.causal ? qb + 1 : n_qb); };
-  const int first = blockIdx.x, stride = gridDim.x;         // heaviest pairs first
+  const int items = fwd_items(n_qb, bh_total, PAIR_ODD);
+  auto item_of = [&](int t) { return FwdItem<PAIR_ODD>(t, n_qb, bh_total, p.causal); };
+  const int first = blockIdx.x, stride = gridDim.x;         // heaviest items first
 
   if (warp == 10) {
     // =========================================================================== TMA producer (+ key bias)
@@ -253,36 +291,41 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     int q_use[2] = {0, 0};
     for (int t = first; t < items; t += stride) {
       if (__shfl_sync(0xffffffffu, lane == 0 ? *abort_flag : 0, 0)) break;     // one decision for the whole warp
-      const int qb0 = 2 * (n_pair - 1 - t / bh_total), bh = t % bh_total;
-      const int h = bh % p.H, b = bh / p.H;
-      const int n_kv = max(n_kv_of(qb0), n_kv_of(qb0 + 1));
+      const auto item = item_of(t);
+      const int b0 = item.bh[0] / p.H, h0 = item.bh[0] - b0 * p.H;
+      const bool wrap = h0 + 1 == p.H;             // the next head is the next sequence's first
+      const int b1 = item.solo && wrap ? b0 + 1 : b0, h1 = item.solo ? (wrap ? 0 : h0 + 1) : h0;
       bool ok = true;
 #pragma unroll
       for (int w = 0; w < 2; ++w) {
-        if (qb0 + w >= n_qb) continue;
+        if (item.n[w] == 0) continue;
         if (lane == 0 && ok) {
           ok = mbar_wait_ol(&bars->q_empty[w], (q_use[w] & 1) ^ 1, abort_flag, p.status, t);
           if (ok) {
             mbar_expect_tx(&bars->q_full[w], kImg);
-            tma_tile<NB>(q_img + w * kImg, &map_q, &bars->q_full[w], (qb0 + w) * kBlk, h, b);
+            tma_tile<NB>(q_img + w * kImg, &map_q, &bars->q_full[w], item.qb[w] * kBlk, w == 0 ? h0 : h1, w == 0 ? b0 : b1);
           }
         }
         ++q_use[w];
       }
-      for (int j = 0; j < n_kv; ++j) {
+      for (int i = 0; i < item.blocks; ++i) {
+        const int j = item.solo ? i >> 1 : i;
+        const int h = i & 1 ? h1 : h0, b = i & 1 ? b1 : b0;        // (the same unless solo)
         const int ks = kv % kFwdRing, kp = (kv / kFwdRing) & 1;
         if (lane == 0) ok = ok && mbar_wait_ol(&bars->kv_empty[ks], kp ^ 1, abort_flag, p.status, t);
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
         if (p.key_bias != nullptr) {
-          // slot j % 4 was last read for block j - 4; both groups were done with block j - 3 before this stage became free
+          // This slot was last read for ring block x - 8.  The stage is free, so the scores of blocks x - 2 and x - 3 have been issued;
+          // each lane has one of the two, and before it handed back the scores of its block before (x - 5 at the earliest): it is
+          // done with those before that.
           float* dst = s_bias + (kcount % kFwdBiasRing) * kBlk;
           bool nz = false;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int key = j * kBlk + lane * 4 + i;
+          for (int e = 0; e < 4; ++e) {
+            const int key = j * kBlk + lane * 4 + e;
             const float v = key < p.T ? p.key_bias[static_cast<int64_t>(b) * p.T + key] * kLog2e : 0.f;
-            dst[lane * 4 + i] = v;
+            dst[lane * 4 + e] = v;
             nz = nz || v != 0.f;
           }
           // an all-zero bias (no padding in this key block) lets the softmax warps skip it
@@ -311,8 +354,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const uint32_t idesc_s = make_idesc_f16(kBlk, kBlk, false, false, p.is_bf16);
     const uint32_t idesc_o = make_idesc_f16(kBlk, DP, false, true, p.is_bf16);
     auto wait = [&](uint64_t* bar, int use, int detail) { return mbar_wait_ol(bar, use & 1, abort_flag, p.status, detail); };
-    // S_w from the K block in ring use `st`
-    auto issue_s = [&](int w, int st, bool last_use, bool last_block, int t) -> bool {
+    // S_w from the K block in ring use `st`; `frees`: arrivals that this lane owes the stage
+    auto issue_s = [&](int w, int st, int frees, bool last_block, int t) -> bool {
       const int ks = st % kFwdRing;
       if (!wait(&bars->kv_full[ks], st / kFwdRing, t)) return false;
       tc_fence_after();
@@ -321,12 +364,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         tc_mma_f16(tmem + w * 128, kmajor_desc(smem_u32(q_img + w * kImg), k16), kmajor_desc(smem_u32(kv_img + ks * kImg), k16),
                    idesc_s, k16 > 0);
       tc_commit(&bars->s_full[w]);
-      if (last_use) tc_commit(&bars->kv_empty[ks]);
+      if (frees > 0) tc_commit(&bars->kv_empty[ks]);
+      if (PAIR_ODD && frees > 1) tc_commit(&bars->kv_empty[ks]);
       if (last_block) tc_commit(&bars->q_empty[w]);
       return true;
     };
     // O_w (+)= P_w V with the V block in ring use `st`, once the group has handed over P_w
-    auto issue_pv = [&](int w, int st, int p_use, bool first_block, bool last_use, int t) -> bool {
+    auto issue_pv = [&](int w, int st, int p_use, bool first_block, int frees, int t) -> bool {
       const int vs = st % kFwdRing;
       if (!wait(&bars->p_ready[w], p_use, t) || !wait(&bars->kv_full[vs], st / kFwdRing, t)) return false;
       const uint32_t tm_o = tmem + 256 + w * (kOwnP ? 64 : 128), tm_p = kOwnP ? tmem + 384 + w * 64 : tmem + w * 128;
@@ -336,7 +380,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         tc_mma_f16_ts(tm_o, tm_p + k16 * 8, mnmajor_desc(smem_u32(kv_img + vs * kImg), k16), idesc_o,
                       (!first_block || k16 > 0) ? 1u : 0u);
       tc_commit(&bars->o_full[w]);
-      if (last_use) tc_commit(&bars->kv_empty[vs]);
+      if (frees > 0) tc_commit(&bars->kv_empty[vs]);
+      if (PAIR_ODD && frees > 1) tc_commit(&bars->kv_empty[vs]);
       return true;
     };
     int kv = 0;                                    // ring uses before this item
@@ -346,52 +391,54 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       const int w = warp - 8;
       int q_use = 0, s_use = 0, p_use = 0;         // uses of q_full / of s_free / of p_ready and o_full
       for (int t = first; t < items && ok && !*abort_flag; t += stride) {
-        const int qb0 = 2 * (n_pair - 1 - t / bh_total);
-        const int n = n_kv_of(qb0 + w), n_kv = max(n_kv_of(qb0), n_kv_of(qb0 + 1));
-        if (n > 0) ok = wait(&bars->q_full[w], q_use++, t) && issue_s(w, kv, true, n == 1, t);
-        for (int j = 0; j < n && ok; ++j) {
-          const int st = kv + 2 * j + 1;
+        const auto item = item_of(t);
+        const int n = w == 0 ? item.n[0] : item.n[1];
+        const int frees = item.solo ? 2 : 1;       // a block of one's own: also the arrival of the lane that does not use it
+        const int step = item.solo ? 4 : 2;
+        int st = kv + (item.solo ? 2 * w : 0);     // K of key block j; V is in the next use
+        if (n > 0) ok = wait(&bars->q_full[w], q_use++, t) && issue_s(w, st, frees, n == 1, t);
+        for (int j = 0; j < n && ok; ++j, st += step) {
           // the group has read S_j for the last time: S_{j+1} goes first, it is what the group needs soonest
           ok = wait(&bars->s_free[w], s_use++, t);
           if (ok && j + 1 < n) {
             tc_fence_after();
-            ok = issue_s(w, st + 1, true, j + 2 == n, t);
+            ok = issue_s(w, st + step, frees, j + 2 == n, t);
           }
-          ok = ok && issue_pv(w, st, p_use++, j == 0, true, t);
+          ok = ok && issue_pv(w, st + 1, p_use++, j == 0, frees, t);
         }
-        // blocks that only the other lane uses: hand them back once they have arrived (earlier would count for an older use)
-        for (int st = kv + 2 * n; st < kv + 2 * n_kv && ok; ++st) {
-          ok = wait(&bars->kv_full[st % kFwdRing], st / kFwdRing, t);
-          if (ok) mbar_arrive(&bars->kv_empty[st % kFwdRing]);
+        // shared blocks that only the other lane uses: hand them back once they have arrived (earlier would count for an older use)
+        for (int u = kv + 2 * n; !item.solo && u < kv + 2 * item.blocks && ok; ++u) {
+          ok = wait(&bars->kv_full[u % kFwdRing], u / kFwdRing, t);
+          if (ok) mbar_arrive(&bars->kv_empty[u % kFwdRing]);
         }
-        kv += 2 * n_kv;
+        kv += 2 * item.blocks;
       }
     } else if (!kOwnP && warp == 8 && lane == 0) {
       // one issuer for both lanes, in turn: that keeps them out of phase, one computing exponentials while the other's
       // products run (with an issuer each they drift into step: 524 us instead of 379 for 4 x 40 heads x 2048 x 128)
       int q_use[2] = {0, 0}, p_use[2] = {0, 0};
       // the next scores lie over P: once P V has finished with it
-      auto next_s = [&](int w, int st, bool last_use, bool last_block, int t) {
-        return (p_use[w] == 0 || wait(&bars->o_full[w], p_use[w] - 1, t)) && issue_s(w, st, last_use, last_block, t);
+      auto next_s = [&](int w, int st, int frees, bool last_block, int t) {
+        return (p_use[w] == 0 || wait(&bars->o_full[w], p_use[w] - 1, t)) && issue_s(w, st, frees, last_block, t);
       };
       for (int t = first; t < items && ok && !*abort_flag; t += stride) {
-        const int qb0 = 2 * (n_pair - 1 - t / bh_total);
-        const int n[2] = {n_kv_of(qb0), n_kv_of(qb0 + 1)};
-        const int n_kv = max(n[0], n[1]);
-        const int last = n[1] > 0 ? 1 : 0;         // the lane that uses every key block, and after the other one
+        const auto item = item_of(t);
+        const int last = item.n[1] > 0 ? 1 : 0;    // the lane that uses every shared key block, and after the other one
+        const int off = item.solo ? 2 : 0, step = item.solo ? 4 : 2;
+        int st = kv;                               // K of lane 0's key block j; lane 1's is `off` uses further, V in the next use
 #pragma unroll
         for (int w = 0; w < 2; ++w)
-          if (ok && n[w] > 0) ok = wait(&bars->q_full[w], q_use[w]++, t) && next_s(w, kv, w == last, n[w] == 1, t);
-        for (int j = 0; j < n_kv && ok; ++j) {
-          const int st = kv + 2 * j + 1;
+          if (ok && item.n[w] > 0)
+            ok = wait(&bars->q_full[w], q_use[w]++, t) && next_s(w, st + w * off, item.solo || w == last, item.n[w] == 1, t);
+        for (int j = 0; j < max(item.n[0], item.n[1]) && ok; ++j, st += step) {
 #pragma unroll
           for (int w = 0; w < 2; ++w) {
-            if (!ok || j >= n[w]) continue;
-            ok = issue_pv(w, st, p_use[w]++, j == 0, w == last, t);
-            if (ok && j + 1 < n[w]) ok = next_s(w, st + 1, w == last, j + 2 == n[w], t);
+            if (!ok || j >= item.n[w]) continue;
+            ok = issue_pv(w, st + w * off + 1, p_use[w]++, j == 0, item.solo || w == last, t);
+            if (ok && j + 1 < item.n[w]) ok = next_s(w, st + w * off + step, item.solo || w == last, j + 2 == item.n[w], t);
           }
         }
-        kv += 2 * n_kv;
+        kv += 2 * item.blocks;
       }
     }
   } else {
@@ -410,10 +457,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if constexpr (kOwnP) attn_trace(threadIdx.x == 0 ? p.trace : nullptr, 0, ntr, code);
     };
     for (int t = first; t < items && ok; t += stride) {
-      const int qb0 = 2 * (n_pair - 1 - t / bh_total), bh = t % bh_total;
-      const int h = bh % p.H, b = bh / p.H;
-      const int qb = qb0 + w, n_kv = n_kv_of(qb);
-      const int item_kv = max(n_kv_of(qb0), n_kv_of(qb0 + 1));
+      const auto item = item_of(t);
+      const int bh = w == 0 ? item.bh[0] : item.bh[1], h = bh % p.H, b = bh / p.H;
+      const int qb = w == 0 ? item.qb[0] : item.qb[1], n_kv = w == 0 ? item.n[0] : item.n[1];
       const int q_idx = qb * kBlk + r;
       float m_run = -INFINITY, l_run = 0.f;
       for (int j = 0; j < n_kv; ++j) {
@@ -425,8 +471,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         const bool tail = k0 + kBlk > p.T;
         const bool cdiag = p.causal && j == qb;
         const bool plain = !tail && !cdiag;
-        const float* bias_j = s_bias + ((kbase + j) % kFwdBiasRing) * kBlk;
-        const bool has_bias = p.key_bias != nullptr && bars->bias_nz[(kbase + j) % kFwdBiasRing] != 0;
+        const int slot = (kbase + (item.solo ? 2 * j + w : j)) % kFwdBiasRing;
+        const float* bias_j = s_bias + slot * kBlk;
+        const bool has_bias = p.key_bias != nullptr && bars->bias_nz[slot] != 0;
         float m_blk = -INFINITY;
         uint32_t ra[32], rb[32];
         // ---- pass 1: the row maximum
@@ -548,7 +595,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         ++use;
       }
       if (!ok) break;
-      kbase += item_kv;
+      kbase += item.blocks;
       if (n_kv == 0) continue;
       // ---- the tile's output: the last P V has landed
       if (!mbar_wait_ol(&bars->o_full[w], (use - 1) & 1, abort_flag, p.status, t)) { ok = false; break; }
@@ -1703,18 +1750,30 @@ struct AttnMaps {
   CUtensorMap dq;   // fp32 dQ accumulator [B*H*T, DP] (persistent backward)
 };
 
-template <typename T, int DP>
-static void launch_fwd(const AttnMaps& m, const AttnParams& p, cudaStream_t s) {
-  auto kern = attn_fwd_kernel<T, DP>;
+template <typename T, int DP, bool PAIR_ODD>
+static void launch_fwd_items(const AttnMaps& m, const AttnParams& p, int items, int sms, cudaStream_t s) {
+  auto kern = attn_fwd_kernel<T, DP, PAIR_ODD>;
   static bool done = false;
   if (!done) {
     C10_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_smem<DP>()));
     done = true;
   }
-  const int items = ((p.T + 2 * kBlk - 1) / (2 * kBlk)) * p.H * p.B;
-  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   kern<<<std::min(items, sms), kFwdThreads, fwd_smem<DP>(), s>>>(m.q, m.k, m.v, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
+}
+template <typename T, int DP>
+static void launch_fwd(const AttnMaps& m, const AttnParams& p, cudaStream_t s) {
+  const int n_qb = (p.T + kBlk - 1) / kBlk, bh_total = p.H * p.B;
+  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  const int items = fwd_items(n_qb, bh_total, false);
+  // Odd last tiles in pairs for more items than CTAs (one tile per head, 64 x 64 heads x 128 tokens, dims of 25 / 32 / 64 / 128: 206 /
+  // 122 / 134 / 169 us with an idle lane, 161 / 89 / 102 / 136 in pairs); up to one item per SM a CTA of its own is sooner done (4 x 4
+  // heads x 384 x 64: 11 and 16).  With three tiles and more it pays for wide heads (64 x 64 heads x 384 x 128: 592 and 517) and
+  // for the padded copies (25: 632 and 587); dims of 32 to 64 are level up to 768 heads and lose beyond (48: 451 and 495).
+  if ((n_qb & 1) && items > sms && (n_qb == 1 || DP > 64 || p.dh % 8 != 0))
+    launch_fwd_items<T, DP, true>(m, p, fwd_items(n_qb, bh_total, true), sms, s);
+  else
+    launch_fwd_items<T, DP, false>(m, p, items, sms, s);
 }
 template <typename T, int DP>
 static void launch_bwd(const AttnMaps& m, const AttnParams& p, cudaStream_t s) {

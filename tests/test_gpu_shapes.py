@@ -93,6 +93,14 @@ def test_layer_norm_refuses_parameters_of_another_length(H):
     (2, 197, 3, 48, False, False),       # the vector row sums with idle lanes
     (2, 70, 3, 24, True, False),         # ... and with four lanes
     (4, 900, 40, 128, True, True),       # several items per CTA
+    (3, 100, 5, 32, True, True),         # one tile per head, fewer than there are SMs
+    (41, 100, 11, 25, True, True),       # ... and more, an odd number: the last has no partner
+    (31, 100, 11, 48, True, True),
+    (30, 128, 12, 80, False, True),
+    (20, 300, 16, 64, False, True),      # an odd last tile alone, then neighbours
+    (10, 300, 17, 25, True, True),       # odd last tiles of two heads, then neighbours
+    (10, 300, 17, 96, False, True),
+    (2, 640, 5, 48, True, True),
 ])
 def test_attention_tiles(dtype, B, T, H, dh, causal, pad):
     ops, ext = _ops()
@@ -104,6 +112,7 @@ def test_attention_tiles(dtype, B, T, H, dh, causal, pad):
     if pad:
         bias = torch.zeros(B, T, device="cuda")
         bias[-1, T // 2:] = -10000.0
+        bias[::3, :T // 5] = -1.5                                 # another bias for every third sequence
     dout = torch.randn(B, T, H * dh, generator=g, device="cuda").to(dtype)
     out = ops.attention_packed(qkv, causal, bias)
     out.backward(dout)
